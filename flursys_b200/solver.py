@@ -14,6 +14,7 @@ from __future__ import annotations
 import ctypes as C
 import dataclasses
 import os
+import threading
 import time
 from dataclasses import dataclass, field
 from typing import Optional
@@ -207,11 +208,13 @@ class Snapshot:
         sizes = (C.c_size_t * len(fids))(*[t.numel() for t in self._host])
         _check(handle.lib, handle.h, handle.lib.flursys_cuda_snapshot_begin(handle.h, ids, len(fids), ptrs, sizes))
         self._done = False
+        self._lock = threading.Lock()  # run() and its writer thread may both wait
 
     def wait(self) -> dict:
-        if not self._done:
-            _check(self._h.lib, self._h.h, self._h.lib.flursys_cuda_snapshot_wait(self._h.h))
-            self._done = True
+        with self._lock:
+            if not self._done:
+                _check(self._h.lib, self._h.h, self._h.lib.flursys_cuda_snapshot_wait(self._h.h))
+                self._done = True
         return {f: t.numpy() for f, t in zip(self.fids, self._host)}
 
 
@@ -492,13 +495,17 @@ class IncompressibleSolver:
             return fu
 
         frame = 0
+        snapshot = None
         while step < self.cfg.max_steps:
             chunk = min(self.cfg.max_steps - step, every - step % every)
             rep = self._h.step(chunk)
             step = int(rep.iteration)
             done = bool(rep.converged) or bool(rep.reached_end_time) or step >= self.cfg.max_steps
             if write_output and (step % every == 0 or done):
-                pending.append(pool.submit(emit, self.field_update_async(), frame))
+                if snapshot is not None:
+                    snapshot.drain()  # a handle holds one; the writer may not have come to it yet
+                snapshot = self.field_update_async()
+                pending.append(pool.submit(emit, snapshot, frame))
                 frame += 1
             if rep.converged:
                 converged = True
@@ -561,6 +568,10 @@ class PendingFieldUpdate:
     def __init__(self, solver: "IncompressibleSolver", snap: Snapshot):
         self._solver = solver
         self._snap = snap
+
+    def drain(self) -> None:
+        """Returns once the fields are in host memory."""
+        self._snap.wait()
 
     def wait(self) -> FieldUpdate:
         f = self._snap.wait()
