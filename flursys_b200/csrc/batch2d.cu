@@ -15,8 +15,10 @@
 //   predict, bnd, rhs  persistent kernels over a table of tiles
 //                      (instance, first element); tiles of stopped instances
 //                      are skipped
-//   pcg2d              one cooperative launch, each instance on its own block
-//                      range with its own bounded barrier (pcg2d.cu)
+//   pcg2d              resident clusters that take the PCG instances off a
+//                      queue, largest first (pcg2d_res.cu); SOR instances and
+//                      those too large for a cluster: one cooperative launch,
+//                      each instance on its own block range (pcg2d.cu)
 //   correct, bnd, post persistent tile kernels as above; post leaves one
 //                      partial record per tile
 //   batch_end          one block per instance: fixed-order reduction of its
@@ -48,6 +50,7 @@
 #include "common.cuh"
 #include "flursys_cuda.h"
 #include "pcg2d.cuh"
+#include "pcg2d_res.cuh"
 
 namespace flursys {
 
@@ -100,7 +103,7 @@ __device__ void share_pressure_blocks(const BatchCtl *ctl, Pcg2dInstance *pin, i
     double wsum = 0.0;
     int nact = 0;
     for (int t = 0; t < n; ++t) {
-        if (!ctl[t].active) continue;
+        if (!ctl[t].active || pin[t].resident) continue;
         const double cells = double(ctl[t].cells);
         const double its = ctl[t].last_iters > 0 ? double(ctl[t].last_iters) : 4.0 * sqrt(cells);
         wsum += cells * its;
@@ -110,7 +113,8 @@ __device__ void share_pressure_blocks(const BatchCtl *ctl, Pcg2dInstance *pin, i
     int b0 = 0;
     for (int t = 0; t < n; ++t) {
         pin[t].block0 = b0;
-        if (!ctl[t].active) {
+        if (pin[t].resident) pin[t].resident = ctl[t].active ? 1 : -1;
+        if (!ctl[t].active || pin[t].resident) {
             pin[t].nblocks = 0;
             continue;
         }
@@ -137,7 +141,8 @@ __global__ void batch_prepare_pressure(const BatchCtl *ctl, Pcg2dInstance *pin, 
     if (threadIdx.x == 0) share_pressure_blocks(ctl, pin, n, total_blocks);
 }
 
-__global__ void batch_begin(BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_blocks) {
+__global__ void batch_begin(BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_blocks, unsigned *queue_next) {
+    if (threadIdx.x == 0) *queue_next = 0u;
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         BatchCtl &c = ctl[t];
         for (int f = 0; f < 4; ++f) c.s.diag->bad_index[f] = ~0ull;
@@ -310,6 +315,10 @@ struct FlursysBatchHandle {
     int tile_elems[kNumOps] = {};
     int grid[kNumOps] = {};
     int pcg_blocks = 0, pcg_per_sm = 0, pcg_max_per_sm = 0;
+    Pcg2dQueuePlan queue;           // resident clusters that solve `queued` of the instances
+    int queued = 0;
+    int *queue_order = nullptr;     // device: their indices, largest first
+    unsigned *queue_next = nullptr; // device
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int graph_nodes = 0;
@@ -406,12 +415,14 @@ cudaError_t set_tiles(FlursysBatchHandle *h, int op, int elems) {
 }
 
 cudaError_t enqueue_step(FlursysBatchHandle *h, cudaStream_t st) {
-    batch_begin<<<1, kBlk, 0, st>>>(h->ctl, h->pin, h->n, h->pcg_blocks);
+    batch_begin<<<1, kBlk, 0, st>>>(h->ctl, h->pin, h->n, h->pcg_blocks, h->queue_next);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = launch_op(h, kOpPredict, st);
     if (e == cudaSuccess) e = launch_op(h, kOpBndStar, st);
     if (e == cudaSuccess) e = launch_op(h, kOpRhs, st);
-    if (e == cudaSuccess) e = pcg2d_launch(h->pin, h->n, h->pcg_blocks, h->precision, st);
+    if (e == cudaSuccess && h->queued)
+        e = pcg2d_queue_launch(h->queue, h->pin, h->queue_order, h->queued, h->queue_next, h->precision, st);
+    if (e == cudaSuccess && h->queued < h->n) e = pcg2d_launch(h->pin, h->n, h->pcg_blocks, h->precision, st);
     if (e == cudaSuccess) e = launch_op(h, kOpCorrect, st);
     if (e == cudaSuccess) e = launch_op(h, kOpBndNew, st);
     if (e == cudaSuccess) e = launch_op(h, kOpPost, st);
@@ -455,6 +466,7 @@ cudaError_t autotune(FlursysBatchHandle *h) {
         if (e == cudaSuccess) e = set_tiles(h, op, best);
     }
     if (e != cudaSuccess) return e;
+    if (h->queued == h->n) return cudaStreamSynchronize(h->stream);  // the resident clusters have nothing to tune
     // pressure kernel: blocks per SM on a synthetic right-hand side, with the
     // iteration caps scaled like the expected iteration counts
     std::vector<Pcg2dInstance> tune = h->h_pin;
@@ -596,6 +608,8 @@ extern "C" int32_t flursys_cuda_batch_create(const FlursysCudaConfig *configs, i
     const size_t res_off = take(sizeof(PcgResultDev) * count);
     const size_t rep_off = take(sizeof(FlursysStepReport) * count);
     const size_t err_off = take(sizeof(unsigned));
+    const size_t order_off = take(sizeof(int) * count);
+    const size_t next_off = take(sizeof(unsigned));
     h->pool_bytes = pos;
     e = cudaMalloc(&h->pool, pos);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->pool, 0, pos, h->stream);
@@ -609,6 +623,8 @@ extern "C" int32_t flursys_cuda_batch_create(const FlursysCudaConfig *configs, i
     h->res = reinterpret_cast<PcgResultDev *>(P + res_off);
     h->rep = reinterpret_cast<FlursysStepReport *>(P + rep_off);
     h->dev_err = reinterpret_cast<unsigned *>(P + err_off);
+    h->queue_order = reinterpret_cast<int *>(P + order_off);
+    h->queue_next = reinterpret_cast<unsigned *>(P + next_off);
     h->h_ctl.assign(count, BatchCtl{});
     h->h_pin.assign(count, Pcg2dInstance{});
     for (int i = 0; i < count && e == cudaSuccess; ++i) {
@@ -689,6 +705,25 @@ extern "C" int32_t flursys_cuda_batch_create(const FlursysCudaConfig *configs, i
         if (e == cudaSuccess) e = cudaMemcpyAsync(s.u, cs.u.data(), 8 * cs.u.size(), cudaMemcpyHostToDevice, h->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(s.v, cs.v.data(), 8 * cs.v.size(), cudaMemcpyHostToDevice, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);  // the host vectors of this case go out of scope later
+    }
+    // PCG instances whose state fits a cluster's shared memory and registers go
+    // to the resident queue, largest first (a long solve taken last would leave
+    // the other clusters idle); the rest share the cooperative launch.
+    std::vector<int> order;
+    if (e == cudaSuccess) {
+        size_t smem = 0, need = 0;
+        for (int i = 0; i < count; ++i)
+            if (h->h_pin[i].solver == FLURSYS_PRESSURE_PCG && pcg2d_queue_fits(h->nx[i], h->ny[i], h->h_pin[i].count_fluid == h->h_ctl[i].cells, h->precision, &need)) {
+                smem = std::max(smem, need);
+                order.push_back(i);
+            }
+        if (!order.empty()) e = pcg2d_queue_plan(h->queue, h->precision, smem, h->device);
+        if (!h->queue.clusters) order.clear();
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->h_ctl[a].cells > h->h_ctl[b].cells; });
+        for (int i : order) h->h_pin[i].resident = 1;
+        h->queued = (int)order.size();
+        if (e == cudaSuccess && h->queued)
+            e = cudaMemcpyAsync(h->queue_order, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, h->stream);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->ctl, h->h_ctl.data(), sizeof(BatchCtl) * count, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->pin, h->h_pin.data(), sizeof(Pcg2dInstance) * count, cudaMemcpyHostToDevice, h->stream);

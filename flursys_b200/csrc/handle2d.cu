@@ -14,6 +14,7 @@
 #include "capi_internal.cuh"
 #include "cavity2d.cuh"
 #include "pcg2d.cuh"
+#include "pcg2d_res.cuh"
 
 namespace flursys {
 
@@ -137,7 +138,7 @@ struct Handle2D {
     uint8_t *flags = nullptr;
     Pcg2dInstance *inst_dev = nullptr;
     Pcg2dInstance inst{};
-    bool cluster = false;  // the pressure solve runs as one thread-block cluster
+    Pcg2dResPlan res;  // chip-resident pressure PCG, where the state fits
     Diag2Dev *h_diag = nullptr;
     int nblocks = 0;
 };
@@ -395,20 +396,11 @@ int32_t init2d(FlursysCudaHandle *h) {
     long long per_block = 512;
     if (const char *env = std::getenv("FLURSYS_2D_CELLS_PER_BLOCK")) per_block = std::max(1LL, std::atoll(env));
     in.nblocks = (int)std::max(1LL, std::min<long long>(h->pcg.grid, ((long long)nc + per_block - 1) / per_block));
-    // A small system without solid or outlet cells (at most 8 cells per
-    // thread) runs as one thread-block cluster instead: the hardware cluster
-    // barrier replaces the software grid barrier. FLURSYS_2D_CLUSTER=0 keeps
-    // the grid path.
-    {
-        const char *cl_env = std::getenv("FLURSYS_2D_CLUSTER");
-        const int maxc = pcg2d_max_cluster(c.precision);
-        const long long threads = (long long)maxc * pcg2d_block_size();
-        if (!(cl_env && std::strcmp(cl_env, "0") == 0) && fluid == (long long)nc && (long long)nc <= 8 * threads &&
-            maxc <= h->pcg.grid) {
-            h2->cluster = true;
-            in.nblocks = (int)std::max(1LL, std::min<long long>(maxc, ((long long)nc + pcg2d_block_size() - 1) /
-                                                                          pcg2d_block_size()));
-        }
+    // PCG keeps its state on the chip where it fits (pcg2d_res.cu).
+    if (c.pressure_solver != FLURSYS_PRESSURE_SOR) {
+        e = pcg2d_res_plan(h2->res, nx, ny, fluid == (long long)nc, c.precision, h->device);
+        if (e != cudaSuccess) return set_cuda_error(&h->err, e, "planning the 2D pressure solve");
+        if (h2->res.enabled) in.nblocks = h2->res.nblocks;
     }
     in.partials = h->pcg.partials;
     in.barrier = h->pcg.barrier;
@@ -433,6 +425,7 @@ void free2d(FlursysCudaHandle *h) {
     cudaFree(h2->flags);
     cudaFree(h2->s.diag);
     cudaFree(h2->inst_dev);
+    pcg2d_res_destroy(h2->res);
     if (h2->h_diag) cudaFreeHost(h2->h_diag);
     delete h2;
     h->h2 = nullptr;
@@ -473,10 +466,12 @@ int32_t step2d(FlursysCudaHandle *h, FlursysStepReport *rep) {
     }
     if (e == cudaSuccess) e = cavity2d_rhs(s, s.rho / (relax * step_dt), st);
     if (e == cudaSuccess) e = cudaEventRecord(h->ev[1], st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(h->pcg.barrier, 0, sizeof(GridBarrier), st);
-    if (e == cudaSuccess)
-        e = h2->cluster ? pcg2d_launch_cluster(h2->inst_dev, h2->inst.nblocks, c.precision, st)
-                        : pcg2d_launch(h2->inst_dev, 1, h2->inst.nblocks, c.precision, st);
+    if (h2->res.enabled) {
+        if (e == cudaSuccess) e = pcg2d_res_launch(h2->res, h2->inst_dev, h->pcg.result, st);
+    } else {
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->pcg.barrier, 0, sizeof(GridBarrier), st);
+        if (e == cudaSuccess) e = pcg2d_launch(h2->inst_dev, 1, h2->inst.nblocks, c.precision, st);
+    }
     if (e == cudaSuccess) e = cudaEventRecord(h->ev[2], st);
     if (e == cudaSuccess) e = cavity2d_correct(s, relax * step_dt / s.rho, st);
     if (simple && e == cudaSuccess) e = cavity2d_simple_relax(s, c.pressure_relaxation, st);
@@ -627,9 +622,16 @@ int32_t stencil_pcg2d(int64_t nx, int64_t ny, double dx, double dy, const double
     in.solver = FLURSYS_PRESSURE_PCG; in.stop_rule = FLURSYS_STOP_REL_L2;
     in.atol = o->absolute_tolerance; in.rtol = o->relative_tolerance;
     in.max_iters = o->max_iterations; in.replace_every = 50;
+    Pcg2dResPlan res;
+    if (e == cudaSuccess) e = pcg2d_res_plan(res, (int)nx, (int)ny, true, precision, device);
+    if (res.enabled) in.nblocks = res.nblocks;
     if (e == cudaSuccess) e = cudaMemcpyAsync(idev, &in, sizeof in, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ws.barrier, 0, sizeof(GridBarrier), st);
-    if (e == cudaSuccess) e = pcg2d_launch(idev, 1, ws.grid, precision, st);
+    if (res.enabled) {
+        if (e == cudaSuccess) e = pcg2d_res_launch(res, idev, ws.result, st);
+    } else {
+        if (e == cudaSuccess) e = cudaMemsetAsync(ws.barrier, 0, sizeof(GridBarrier), st);
+        if (e == cudaSuccess) e = pcg2d_launch(idev, 1, ws.grid, precision, st);
+    }
     if (e == cudaSuccess) e = cudaMemcpyAsync(ws.h_result, ws.result, sizeof(PcgResultDev), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(x_inout, dxp, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -644,6 +646,7 @@ int32_t stencil_pcg2d(int64_t nx, int64_t ny, double dx, double dy, const double
         report->final_residual = r.residual;
         report->relative_residual = r.initial == 0.0 ? 0.0 : r.residual / r.initial;
     }
+    pcg2d_res_destroy(res);
     ws.free_all();
     cudaFree(dxp);
     cudaFree(drhs);

@@ -44,15 +44,8 @@ constexpr int kRoundCols = 8;
 constexpr int kParts = 2 * kRoundCols;
 constexpr int kU = 4;  // cells per thread per step of the plain-operator passes
 
-// Barriers between the passes of one instance. GridSync: the bounded
-// software grid barrier over the instance's blocks. ClusterSync: the
-// instance runs as one thread-block cluster and the passes are separated by
-// the hardware cluster barrier (release / acquire at cluster scope, so
-// everything written before it is visible after it in every block of the
-// cluster). Either way the blocks' partial sums meet in global memory, read
-// through L2. (Partials in distributed shared memory measured no faster on
-// the 128^2 cavity and need a closing barrier to keep every block's shared
-// memory alive until the last read.)
+// Barriers between the passes of one instance: the bounded software grid
+// barrier over the instance's blocks.
 struct GridSync {
     GridBarrier *bar;
     unsigned nb;
@@ -62,16 +55,6 @@ struct GridSync {
     __device__ __forceinline__ void put(int lb, int col, double v) const { partials[lb * kParts + col] = v; }
     __device__ __forceinline__ double get(int b, int col) const { return __ldcg(partials + b * kParts + col); }
 };
-struct ClusterSync {
-    double *partials;
-    __device__ __forceinline__ bool operator()() const {
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        return true;
-    }
-    __device__ __forceinline__ void put(int lb, int col, double v) const { partials[lb * kParts + col] = v; }
-    __device__ __forceinline__ double get(int b, int col) const { return __ldcg(partials + b * kParts + col); }
-};
-
 __device__ __forceinline__ bool solid(const uint8_t *f, int c) { return (f[c] & kCellSolid) != 0; }
 __device__ __forceinline__ bool ident(const uint8_t *f, int c) { return (f[c] & 3) != 0; }
 
@@ -642,18 +625,6 @@ __global__ void __launch_bounds__(kBlock, 3) pcg2d_kernel(const Pcg2dInstance *_
     else pcg_instance<V, MIXED>(k, red, sync);
 }
 
-// One instance as one thread-block cluster (grid = cluster = nblocks): the
-// passes are separated by the hardware cluster barrier.
-template <typename V, bool MIXED>
-__global__ void __launch_bounds__(kBlock, 3) pcg2d_cluster_kernel(const Pcg2dInstance *__restrict__ inst) {
-    __shared__ double red[kRoundCols * (kBlock / 32)];
-    Ctx k;
-    make_ctx(k, inst[0], (int)blockIdx.x);
-    const ClusterSync sync{k.in.partials};
-    if (k.in.solver == FLURSYS_PRESSURE_SOR) sor_instance(k, red, sync);
-    else pcg_instance<V, MIXED>(k, red, sync);
-}
-
 }  // namespace
 
 cudaError_t pcg2d_max_grid(int precision, int device, int *grid) {
@@ -667,48 +638,6 @@ cudaError_t pcg2d_max_grid(int precision, int device, int *grid) {
     if (e != cudaSuccess) return e;
     *grid = sms * per_sm;
     return cudaSuccess;
-}
-
-int pcg2d_max_cluster(int precision) {
-    const void *fn = precision == FLURSYS_PRECISION_MIXED ? (const void *)pcg2d_cluster_kernel<float, true>
-                                                          : (const void *)pcg2d_cluster_kernel<double, false>;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-        cudaGetLastError();
-        return 8;  // the portable cluster size
-    }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(kBlock);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 16;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int size = 0;
-    if (cudaOccupancyMaxPotentialClusterSize(&size, fn, &cfg) != cudaSuccess || size < 1) {
-        cudaGetLastError();
-        return 8;
-    }
-    return size;
-}
-
-cudaError_t pcg2d_launch_cluster(const Pcg2dInstance *inst_dev, int nblocks, int precision, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(nblocks);
-    cfg.blockDim = dim3(kBlock);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = nblocks;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (precision == FLURSYS_PRECISION_MIXED) return cudaLaunchKernelEx(&cfg, pcg2d_cluster_kernel<float, true>, inst_dev);
-    return cudaLaunchKernelEx(&cfg, pcg2d_cluster_kernel<double, false>, inst_dev);
 }
 
 int pcg2d_block_size() { return kBlock; }
