@@ -35,6 +35,16 @@ struct PcgWorkspace {
 
 struct Handle2D;
 
+// How a 3D handle's SOR runs (sor.cu): blocks == 0 streams p through L2.
+struct RedRecord;
+struct Sor3dPlan {
+    int blocks = 0;
+    bool cluster = false;
+    size_t smem = 0;
+    RedRecord *records = nullptr;
+    unsigned epoch = 0;
+};
+
 }  // namespace flursys
 
 struct FlursysCudaHandle {
@@ -53,6 +63,7 @@ struct FlursysCudaHandle {
     flursys::PcgWorkspace pcg;
     flursys::Pcg3dSeqPlan seq;   // graph-driven PCG (default 3D PCG path)
     bool use_seq = false;
+    flursys::Sor3dPlan sor;
     flursys::CgSeqState *h_seq = nullptr;  // pinned host copy of the solve state
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     // 2D state

@@ -71,6 +71,10 @@ static int32_t init3d(FlursysCudaHandle *h) {
         if (st) return st;
         return FLURSYS_OK;
     }
+    if (c.pressure_solver == FLURSYS_PRESSURE_SOR) {
+        e = sor3d_plan(h->sor, s.nx, s.ny, s.nz, h->device);
+        if (e != cudaSuccess) return set_cuda_error(&h->err, e, "planning the SOR solve");
+    }
     // The graph-driven PCG is the default; FLURSYS_PCG_VARIANT=persistent
     // selects the single cooperative kernel instead.
     const char *variant = std::getenv("FLURSYS_PCG_VARIANT");
@@ -114,6 +118,7 @@ void handle_free(FlursysCudaHandle *h) {
     if (h->h_diag3) cudaFreeHost(h->h_diag3);
     h->pcg.free_all();
     pcg3d_seq_destroy(h->seq);
+    sor3d_destroy(h->sor);
     if (h->fcg_net) fcgnet_destroy(h->fcg_net);
     h->fcg_net = nullptr;
     if (h->h_seq) cudaFreeHost(h->h_seq);
@@ -150,7 +155,7 @@ int32_t step3d(FlursysCudaHandle *h, FlursysStepReport *rep) {
             m.initial_l2 = f.initial_residual;
         }
     } else if (sor) {
-        status = run_sor3d(h->pcg, s.nx, s.ny, s.nz, s.dx, s.dy, s.dz, s.p, s.rhs, c.pressure_omega,
+        status = run_sor3d(h->sor, h->pcg, s.nx, s.ny, s.nz, s.dx, s.dy, s.dz, s.p, s.rhs, c.pressure_omega,
                            c.pressure_tolerance, c.pressure_max_iters, st, &h->err);
     } else if (h->use_seq) {
         const cudaError_t le = pcg3d_seq_launch(h->seq, st);
