@@ -21,8 +21,9 @@
 //   conv_last   16 -> 1 channel (FP32 output, CUDA cores, staged tile; training)
 //   net_in_fused / net_out_interior + net_out_boundary  the full-resolution layers of inference,
 //               collapsed by linearity into composite stencils (see below)
-//   wgrad       dW[co][tap][ci] += sum_v dY[v][co] X[v + tap][ci] (CUDA cores,
-//               FP32, atomics per voxel chunk)
+//   wgrad_mma   dW[co][tap][ci] += sum_v dY[v][co] X[v + tap][ci] of the BF16
+//               layers (mma.sync, FP32); wgrad_scalar of the layers with one
+//               channel on one side (CUDA cores, FP32)
 // The data gradient of a layer is the forward convolution with the
 // transposed, flipped weights (NetWeights::bwd), so conv_tc serves both.
 #include <cuda_bf16.h>
@@ -486,41 +487,200 @@ __global__ void upadd_kernel(const uint16_t *coarse, const uint16_t *skip, uint1
     }
 }
 
-template <typename T>
-__device__ __forceinline__ float ld(const T *p, long long i);
-template <>
-__device__ __forceinline__ float ld<float>(const float *p, long long i) { return p[i]; }
-template <>
-__device__ __forceinline__ float ld<uint16_t>(const uint16_t *p, long long i) { return bf2f(p[i]); }
+// ---- weight gradients ---------------------------------------------------
+// dW[co][tap][ci] += sum over voxels v of dY[v][co] X[v + tap][ci]: for each
+// tap a GEMM with M = COUT, N = CIN and the voxels as K, both operands BF16 as
+// stored (channels innermost, so both come through transposing ldmatrix).
+// A block owns the three taps of one (dz, dy) and marches over its share of
+// the rows, 64 voxel slots at a time; the taps dx are the staged row of X read
+// one voxel apart. A warp owns 16 output channels of one tap. Rows are cut into
+// pieces of at most 64 voxels padded to 16 with zeros, several to a stage where
+// they are short; two stages alternate, the next in flight (cp.async) during
+// the MMAs. Each piece (at most 4 chained MMAs) is summed from zero and added
+// to the FP32 accumulator by the CUDA cores, so that no long chain runs through
+// the tensor cores' own accumulation.
+// One thread per weight, walking 1024 voxels with two dependent loads per
+// product, took 844 us on 64 -> 32 channels at 16^3 and 432 us on 16 -> 32 at
+// 32^3: latency, at 0.5 TFLOP/s.
+constexpr int kWgSlots = 64;                // voxel slots of a stage
+constexpr int kWgXSlots = kWgSlots + 2 * 4;  // with two halo slots for each of at most four pieces
 
-constexpr int kWgradChunk = 1024;
+struct WgradGeom {
+    int nx, ny, nz;
+    int len, padded, pieces, per_stage;  // voxels of a piece, padded to 16; pieces of a row, of a stage
+    long long total, stages;             // pieces and stages in all
+};
 
-// dW[co][tap][ci] += sum over a chunk of voxels v of dY[v][co] * X[v + tap][ci].
-template <typename TX, typename TY>
-__global__ void __launch_bounds__(256) wgrad_kernel(const TX *X, const TY *dY, float *dW, int cin, int cout, int nx,
-                                                    int ny, int nz) {
-    const int per = 27 * cin;
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= cout * per) return;
-    const int co = o / per, rem = o - co * per, tap = rem / cin, ci = rem - tap * cin;
-    const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-    const long long n = (long long)nx * ny * nz;
-    const long long v0 = (long long)blockIdx.y * kWgradChunk;
-    const long long v1 = v0 + kWgradChunk < n ? v0 + kWgradChunk : n;
-    int x = int(v0 % nx);
-    long long t = v0 / nx;
-    int y = int(t % ny), z = int(t / ny);
-    float acc = 0.f;
-    for (long long v = v0; v < v1; ++v) {
-        const int xx = x + dx, yy = y + dy, zz = z + dz;
-        if (xx >= 0 && yy >= 0 && zz >= 0 && xx < nx && yy < ny && zz < nz)
-            acc = fmaf(ld(dY, v * cout + co), ld(X, (((long long)zz * ny + yy) * nx + xx) * cin + ci), acc);
-        if (++x == nx) {
-            x = 0;
-            if (++y == ny) { y = 0; ++z; }
+WgradGeom wgrad_geom(int nx, int ny, int nz) {
+    WgradGeom g{nx, ny, nz};
+    g.pieces = (nx + kWgSlots - 1) / kWgSlots;
+    g.len = (nx + g.pieces - 1) / g.pieces;
+    g.padded = (g.len + 15) / 16 * 16;
+    g.per_stage = kWgSlots / g.padded;
+    g.total = (long long)ny * nz * g.pieces;
+    g.stages = (g.total + g.per_stage - 1) / g.per_stage;
+    return g;
+}
+
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3, const void *p) {
+    const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p));
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "r"(a));
+}
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(6 * COUT) wgrad_mma(const uint16_t *__restrict__ X, const uint16_t *__restrict__ dY,
+                                                      float *dW, const WgradGeom g) {
+    constexpr int kThreads = 6 * COUT;  // 3 taps x COUT / 16 warps
+    constexpr int SY = COUT + kPad, SX = CIN + kPad, NT = CIN / 8;
+    __shared__ __align__(16) uint16_t sY[2][kWgSlots * SY];
+    __shared__ __align__(16) uint16_t sX[2][kWgXSlots * SX];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int dx = warp % 3, co0 = (warp / 3) * 16;  // dx: halo-relative 0..2
+    const int dy = (int)blockIdx.y % 3 - 1, dz = (int)blockIdx.y / 3 - 1;
+
+    auto stage = [&](long long st, int buf) {
+        for (int e = threadIdx.x; e < kWgSlots * (COUT / 8); e += kThreads) {
+            const int k8 = e % (COUT / 8), v = e / (COUT / 8), u = v / g.padded, xi = v - u * g.padded;
+            const long long piece = st * g.per_stage + u, row = piece / g.pieces;
+            const int x = (int)(piece - row * g.pieces) * g.len + xi;
+            const bool ok = u < g.per_stage && piece < g.total && xi < g.len && x < g.nx;
+            cp_async_zfill<16>(&sY[buf][v * SY + k8 * 8], dY + (ok ? (row * g.nx + x) * COUT + k8 * 8 : 0), ok);
         }
+        for (int e = threadIdx.x; e < kWgXSlots * (CIN / 8); e += kThreads) {
+            const int k8 = e % (CIN / 8), v = e / (CIN / 8), u = v / (g.padded + 2), xi = v - u * (g.padded + 2);
+            const long long piece = st * g.per_stage + u, row = piece / g.pieces;
+            const int x = (int)(piece - row * g.pieces) * g.len + xi - 1;
+            const int y = (int)(row % g.ny) + dy, z = (int)(row / g.ny) + dz;
+            const bool ok = u < g.per_stage && piece < g.total && x >= 0 && x < g.nx && y >= 0 && y < g.ny && z >= 0 &&
+                            z < g.nz;
+            cp_async_zfill<16>(&sX[buf][v * SX + k8 * 8],
+                               X + (ok ? (((long long)z * g.ny + y) * g.nx + x) * CIN + k8 * 8 : 0), ok);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
+    // ldmatrix rows: voxel 8 (i >> 1) + r, channel 8 (i & 1) of A's four
+    // matrices i; voxel 8 (i & 1) + r, channel 8 (i >> 1) of two B tiles
+    const int mi = lane >> 3, mr = lane & 7;
+    const int a_off = (8 * (mi >> 1) + mr) * SY + 8 * (mi & 1) + co0;
+    const int b_off = (8 * (mi & 1) + mr + dx) * SX + 8 * (mi >> 1);
+    int buf = 0;
+    if (blockIdx.x < g.stages) stage(blockIdx.x, 0);
+    for (long long st = blockIdx.x; st < g.stages; st += gridDim.x, buf ^= 1) {
+        const bool more = st + gridDim.x < g.stages;
+        if (more) stage(st + gridDim.x, buf ^ 1);
+        if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        for (int u = 0; u < g.per_stage; ++u) {
+            float part[NT][4];
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) part[n][e] = 0.f;
+            const uint16_t *pa = sY[buf] + u * g.padded * SY + a_off, *pb = sX[buf] + u * (g.padded + 2) * SX + b_off;
+            for (int k = 0; k < g.padded; k += 16) {
+                uint32_t a0, a1, a2, a3;
+                ldsm_x4_trans(a0, a1, a2, a3, pa + k * SY);
+#pragma unroll
+                for (int n = 0; n < NT; n += 2) {
+                    uint32_t b0, b1, b2, b3;
+                    ldsm_x4_trans(b0, b1, b2, b3, pb + k * SX + n * 8);
+                    mma_bf16(part[n], a0, a1, a2, a3, b0, b1);
+                    mma_bf16(part[n + 1], a0, a1, a2, a3, b2, b3);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[n][e] += part[n][e];
+        }
+        __syncthreads();
     }
-    atomicAdd(dW + o, acc);
+    const int tap = (dz + 1) * 9 + (dy + 1) * 3 + dx, gr = lane >> 2, tc = 2 * (lane & 3);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            atomicAdd(dW + ((long long)(co0 + gr + 8 * (e >> 1)) * 27 + tap) * CIN + n * 8 + tc + (e & 1), acc[n][e]);
+}
+
+// The layers with one channel on one side: T[c][tap] = sum over voxels u of
+// Y[u][c] S[u + tap], Y the 16-channel BF16 tensor, S the FP32 scalar one.
+// FIRST (1 -> 16): Y = dY, S = X, dW[c][tap]; otherwise (16 -> 1): Y = X, S =
+// dY, dW[26 - tap][c], the tap seen from X. A block stages pieces of 64 voxels
+// of a row with the nine rows of S around it; a thread owns four channels and
+// the three taps dx of one (dz, dy) over an eighth of the piece, S sliding
+// through registers (12 products for two shared loads; one thread per weight
+// took 357 us at 64^3).
+constexpr int kWsLen = 64, kWsGroups = 8, kWsThreads = 36 * kWsGroups;
+
+template <bool FIRST>
+__global__ void __launch_bounds__(kWsThreads) wgrad_scalar(const uint16_t *__restrict__ Y, const float *__restrict__ S,
+                                                           float *dW, int nx, int ny, int nz) {
+    __shared__ float sS[9][kWsLen + 2];
+    __shared__ __align__(16) float sY[kWsLen * 16];
+    __shared__ float sum[kWsGroups][432];
+    const int grp = threadIdx.x / 36, o = threadIdx.x % 36, pair = o >> 2, quad = o & 3;
+    const int pieces = (nx + kWsLen - 1) / kWsLen;
+    const long long total = (long long)ny * nz * pieces;
+    float acc[3][4] = {};
+    for (long long p = blockIdx.x; p < total; p += gridDim.x) {
+        const long long row = p / pieces;
+        const int x0 = (int)(p - row * pieces) * kWsLen, y = (int)(row % ny), z = (int)(row / ny);
+        for (int e = threadIdx.x; e < 9 * (kWsLen + 2); e += kWsThreads) {
+            const int q = e / (kWsLen + 2), x = x0 + e % (kWsLen + 2) - 1, yy = y + q % 3 - 1, zz = z + q / 3 - 1;
+            const bool ok = x >= 0 && x < nx && yy >= 0 && yy < ny && zz >= 0 && zz < nz;
+            sS[q][e % (kWsLen + 2)] = ok ? S[((long long)zz * ny + yy) * nx + x] : 0.f;
+        }
+        for (int e = threadIdx.x; e < kWsLen * 2; e += kWsThreads) {  // eight channels each
+            const int v = e >> 1, x = x0 + v;
+            uint4 t = make_uint4(0, 0, 0, 0);
+            if (x < nx) t = *reinterpret_cast<const uint4 *>(Y + (row * nx + x) * 16 + 8 * (e & 1));
+            const uint16_t *h = reinterpret_cast<const uint16_t *>(&t);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) sY[v * 16 + 8 * (e & 1) + c] = bf2f(h[c]);
+        }
+        __syncthreads();
+        const int v0 = grp * (kWsLen / kWsGroups);
+        float s0 = sS[pair][v0], s1 = sS[pair][v0 + 1];
+#pragma unroll
+        for (int v = v0; v < v0 + kWsLen / kWsGroups; ++v) {
+            const float s2 = sS[pair][v + 2];
+            const float4 yv = *reinterpret_cast<const float4 *>(sY + v * 16 + quad * 4);
+            const float yc[4] = {yv.x, yv.y, yv.z, yv.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                acc[0][c] = fmaf(yc[c], s0, acc[0][c]);
+                acc[1][c] = fmaf(yc[c], s1, acc[1][c]);
+                acc[2][c] = fmaf(yc[c], s2, acc[2][c]);
+            }
+            s0 = s1;
+            s1 = s2;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int tap = pair * 3 + t, ch = quad * 4 + c;
+            sum[grp][FIRST ? ch * 27 + tap : (26 - tap) * 16 + ch] = acc[t][c];
+        }
+    __syncthreads();
+    for (int e = threadIdx.x; e < 432; e += kWsThreads) {
+        float t = 0.f;
+#pragma unroll
+        for (int k = 0; k < kWsGroups; ++k) t += sum[k][e];
+        atomicAdd(dW + e, t);
+    }
 }
 
 // Energy-norm loss of e = out - p_hat on the unit-spacing Neumann operator L:
@@ -658,7 +818,7 @@ constexpr int kFusedCount = kFusedWp + 8 * 8 * 16;
 __global__ void pack_fused(const float *master, long long off_first, long long off_last, float *fz) {
     const float *W1 = master + off_first;  // [16][27][1]
     const float *W7 = master + off_last;   // [1][27][16]
-    for (int i = threadIdx.x; i < kFusedCount; i += blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kFusedCount; i += gridDim.x * blockDim.x) {
         double acc = 0.0;
         if (i < kFusedK125) {  // K2[c][o], o = (oz*4 + oy)*4 + ox
             const int c = i / 64, o = i % 64;
@@ -720,7 +880,7 @@ __device__ __forceinline__ float up_weight(const float *wp, int o, int n, int k)
 
 __global__ void pack_upfrag(const float *fz, uint32_t *upfrag) {
     const float *wp = fz + kFusedWp;
-    for (int i = threadIdx.x; i < kUpFragWords; i += blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kUpFragWords; i += gridDim.x * blockDim.x) {
         const int reg = i & 1, lane = (i >> 1) & 31, split = (i >> 6) & 1, o = i >> 7;
         const int n = lane >> 2, k = 2 * (lane & 3) + 8 * reg;
         uint32_t word = 0;
@@ -745,7 +905,7 @@ constexpr int kInFragWords = 32 * 32;
 
 __global__ void pack_infrag(const float *fz, uint32_t *infrag) {
     const float *k2 = fz + kFusedK2;  // [16 channels][64 taps]
-    for (int i = threadIdx.x; i < kInFragWords; i += blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kInFragWords; i += gridDim.x * blockDim.x) {
         const int lane = i >> 5, w = i & 31;
         const int reg = w & 1, split = (w >> 1) & 1, nt = (w >> 2) & 1, kc = w >> 3;
         const int c = 8 * nt + (lane >> 2), o = 16 * kc + 2 * (lane & 3) + 8 * reg;
@@ -1959,12 +2119,18 @@ cudaError_t upadd_any(int c, const uint16_t *coarse, const uint16_t *skip, uint1
     }
 }
 
-template <typename TX, typename TY>
-cudaError_t launch_wgrad(const TX *X, const TY *dY, float *dW, int cin, int cout, int nx, int ny, int nz,
-                         cudaStream_t st) {
-    const long long n = (long long)nx * ny * nz;
-    dim3 grid((cout * 27 * cin + 255) / 256, (unsigned)((n + kWgradChunk - 1) / kWgradChunk));
-    wgrad_kernel<TX, TY><<<grid, 256, 0, st>>>(X, dY, dW, cin, cout, nx, ny, nz);
+template <int CIN, int COUT>
+cudaError_t launch_wgrad(const uint16_t *X, const uint16_t *dY, float *dW, int nx, int ny, int nz, cudaStream_t st) {
+    const WgradGeom g = wgrad_geom(nx, ny, nz);
+    // nine (dz, dy) blocks per share of the rows: about four blocks per SM at most
+    dim3 grid((unsigned)std::min<long long>(g.stages, 64), 9);
+    wgrad_mma<CIN, COUT><<<grid, 6 * COUT, 0, st>>>(X, dY, dW, g);
+    return cudaGetLastError();
+}
+template <bool FIRST>
+cudaError_t launch_wgrad_scalar(const uint16_t *Y, const float *S, float *dW, int nx, int ny, int nz, cudaStream_t st) {
+    const long long total = (long long)ny * nz * ((nx + kWsLen - 1) / kWsLen);
+    wgrad_scalar<FIRST><<<(unsigned)std::min<long long>(total, 148 * 4), kWsThreads, 0, st>>>(Y, S, dW, nx, ny, nz);
     return cudaGetLastError();
 }
 
@@ -2063,9 +2229,9 @@ void NetWeights::release() {
 cudaError_t net_pack_weights(const float *master, NetWeights &w, cudaStream_t st) {
     const long long n = net_param_count();
     pack_kernel<<<grid_1d(n), 256, 0, st>>>(master, w.fwd, w.bwd, w.fwd_f32, n);
-    pack_fused<<<1, 256, 0, st>>>(master, net_param_offset(0), net_param_offset(kNetLayers - 1), w.fused);
-    pack_upfrag<<<1, 256, 0, st>>>(w.fused, w.upfrag);
-    pack_infrag<<<1, 256, 0, st>>>(w.fused, w.infrag);
+    pack_fused<<<(kFusedCount + 63) / 64, 64, 0, st>>>(master, net_param_offset(0), net_param_offset(kNetLayers - 1), w.fused);
+    pack_upfrag<<<(kUpFragWords + 127) / 128, 128, 0, st>>>(w.fused, w.upfrag);
+    pack_infrag<<<(kInFragWords + 127) / 128, 128, 0, st>>>(w.fused, w.infrag);
     w.host_params_valid = false;
     return cudaGetLastError();
 }
@@ -2176,28 +2342,28 @@ cudaError_t net_train_sample(const NetWeights &w, NetWorkspace &ws, int nx, int 
         e = cudaGetLastError();
     }
     // ---- backward: weight gradient of each layer, then its data gradient ----
-    if (e == cudaSuccess) e = launch_wgrad<uint16_t, float>(ws.x7, ws.gout, grad + off(6), 16, 1, nx, ny, nz, st);
+    if (e == cudaSuccess) e = launch_wgrad_scalar<false>(ws.x7, ws.gout, grad + off(6), nx, ny, nz, st);
     if (e == cudaSuccess) {
         conv_first<<<grid_1d(n), 256, 0, st>>>(ws.gout, w.fwd_f32 + 864, nullptr, ws.g7, nullptr, nx, ny, nz);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = pool_any(16, ws.g7, ws.gb2, n2x, n2y, n2z, 1.f, st);
-    if (e == cudaSuccess) e = launch_wgrad<uint16_t, uint16_t>(ws.x6, ws.gb2, grad + off(5), 32, 16, n2x, n2y, n2z, st);
+    if (e == cudaSuccess) e = launch_wgrad<32, 16>(ws.x6, ws.gb2, grad + off(5), n2x, n2y, n2z, st);
     if (e == cudaSuccess) e = launch_conv<16, 32, kPlain>(Src{ws.gb2, nullptr}, Wb + off(5), ws.g6, n2x, n2y, n2z, st);
     if (e == cudaSuccess) e = pool_any(32, ws.g6, ws.gb3, n3x, n3y, n3z, 1.f, st);
-    if (e == cudaSuccess) e = launch_wgrad<uint16_t, uint16_t>(ws.x5, ws.gb3, grad + off(4), 64, 32, n3x, n3y, n3z, st);
+    if (e == cudaSuccess) e = launch_wgrad<64, 32>(ws.x5, ws.gb3, grad + off(4), n3x, n3y, n3z, st);
     if (e == cudaSuccess) e = launch_conv<32, 64, kPlain>(Src{ws.gb3, nullptr}, Wb + off(4), ws.g5, n3x, n3y, n3z, st);
     if (e == cudaSuccess) e = pool_any(64, ws.g5, ws.ga4, n4x, n4y, n4z, 1.f, st);
-    if (e == cudaSuccess) e = launch_wgrad<uint16_t, uint16_t>(ws.x4, ws.ga4, grad + off(3), 64, 64, n4x, n4y, n4z, st);
+    if (e == cudaSuccess) e = launch_wgrad<64, 64>(ws.x4, ws.ga4, grad + off(3), n4x, n4y, n4z, st);
     if (e == cudaSuccess) e = launch_conv<64, 64, kPlain>(Src{ws.ga4, nullptr}, Wb + off(3), ws.g4, n4x, n4y, n4z, st);
     if (e == cudaSuccess) e = upadd_any(64, ws.g4, ws.ga3, ws.ga3, n3x, n3y, n3z, 0.125f, 1, st);
-    if (e == cudaSuccess) e = launch_wgrad<uint16_t, uint16_t>(ws.x3, ws.ga3, grad + off(2), 32, 64, n3x, n3y, n3z, st);
+    if (e == cudaSuccess) e = launch_wgrad<32, 64>(ws.x3, ws.ga3, grad + off(2), n3x, n3y, n3z, st);
     if (e == cudaSuccess) e = launch_conv<64, 32, kPlain>(Src{ws.ga3, nullptr}, Wb + off(2), ws.g3, n3x, n3y, n3z, st);
     if (e == cudaSuccess) e = upadd_any(32, ws.g3, ws.ga2, ws.ga2, n2x, n2y, n2z, 0.125f, 1, st);
-    if (e == cudaSuccess) e = launch_wgrad<uint16_t, uint16_t>(ws.x2, ws.ga2, grad + off(1), 16, 32, n2x, n2y, n2z, st);
+    if (e == cudaSuccess) e = launch_wgrad<16, 32>(ws.x2, ws.ga2, grad + off(1), n2x, n2y, n2z, st);
     if (e == cudaSuccess) e = launch_conv<32, 16, kPlain>(Src{ws.ga2, nullptr}, Wb + off(1), ws.g2, n2x, n2y, n2z, st);
     if (e == cudaSuccess) e = upadd_any(16, ws.g2, ws.ga1, ws.ga1, nx, ny, nz, 0.125f, 1, st);
-    if (e == cudaSuccess) e = launch_wgrad<float, uint16_t>(b_hat, ws.ga1, grad + off(0), 1, 16, nx, ny, nz, st);
+    if (e == cudaSuccess) e = launch_wgrad_scalar<true>(ws.ga1, b_hat, grad + off(0), nx, ny, nz, st);
     return e;
 }
 
