@@ -169,6 +169,7 @@ struct GridGroup {
     unsigned epoch;
     long long spin_limit;
     bool fault;                   // injected: every wait gives up at once
+    bool plain_faces = false;     // faces are plain global stores, ordered by the round's fences
 
     __device__ __forceinline__ unsigned long long tag(unsigned r) const {
         return ((unsigned long long)epoch << 32) | (unsigned long long)(r + 1u);
@@ -218,6 +219,7 @@ struct GridGroup {
         ++round;
         if (wid == 0) {
             const double t = rows_reduce8(sm->warp, T / 32, max7);
+            if (plain_faces && with_faces) asm volatile("fence.acq_rel.gpu;" ::: "memory");
             if ((lane & 3) == 0) st_record(set + (size_t)rank * kRedSlots + (lane >> 2), t, want);
         }
         // value threadIdx & 7 of blocks threadIdx / 8 + i * T / 8; a record
@@ -246,6 +248,7 @@ struct GridGroup {
                 break;
             }
         }
+        if (plain_faces && with_faces) asm volatile("fence.acq_rel.gpu;" ::: "memory");
         look();
         const bool m = max7 && (threadIdx.x & 7) == 7;
         double t = 0.0;
@@ -311,6 +314,7 @@ struct ClusterGroup {
     int nb, rank, face_slots;
     unsigned round, fround;
     uint32_t faces;  // shared address of this block's 2 * face_slots face values
+    bool fault = false;  // injected: the first reduction gives up
 
     __device__ __forceinline__ void init() {
         if (threadIdx.x == 0) {
@@ -370,6 +374,7 @@ struct ClusterGroup {
     // block barrier that warp 0 enters afterwards orders the faces for them.
     template <typename F>
     __device__ __forceinline__ bool lead(double (&v)[kRedSlots], bool max7, bool with_faces, unsigned face_bytes, F) {
+        if (fault) return false;
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
         const double w = warp_reduce8(v, max7);
         if ((lane & 3) == 0) sm->warp[wid * kRedSlots + (lane >> 2)] = w;

@@ -34,6 +34,7 @@
 #include "pcg3d.cuh"
 #include "pcg3d_seq.cuh"
 #include "pcg3d_res.cuh"
+#include "pcg3d_rows.cuh"
 #include "tma.cuh"
 
 namespace flursys {
@@ -1819,9 +1820,18 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
     plan.host_args = new SeqArgs(a);
     const char *v = std::getenv("FLURSYS_PCG_VARIANT");
     if (v && std::strcmp(v, "host") == 0) plan.host_iterations = 1;
-    // MIXED solves whose tiles fit one per SM run chip-resident (one
-    // cooperative launch per solve; FLURSYS_PCG_RESIDENT=0 keeps the graph).
-    if (e == cudaSuccess && precision == FLURSYS_PRECISION_MIXED && !a.cg1 && plan.host_iterations == 0) {
+    // Solves whose rows fit the chip run resident, one launch per solve, F64
+    // and MIXED (pcg3d_rows.cu: less per iteration than every other form at all
+    // sizes that it holds). MIXED grids between that and one 32 x 32 x tz tile
+    // per SM (192 x 128 x 96) keep the tile-resident form (pcg3d_res.cu).
+    // FLURSYS_PCG_RESIDENT=0 keeps the graph, =2 the tile-resident form.
+    if (e == cudaSuccess && !a.cg1 && plan.host_iterations == 0) {
+        auto *rp = new Pcg3dRowsPlan();
+        if (pcg3d_rows_plan(*rp, args, precision, device)) plan.rows = rp;
+        else delete rp;
+        cudaGetLastError();  // a declined plan leaves no sticky error behind
+    }
+    if (e == cudaSuccess && !plan.rows && precision == FLURSYS_PRECISION_MIXED && !a.cg1 && plan.host_iterations == 0) {
         auto *rp = new Pcg3dResPlan();
         if (pcg3d_res_plan(*rp, args, device)) plan.resident = rp;
         else delete rp;
@@ -1831,6 +1841,7 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
 }
 
 cudaError_t pcg3d_seq_launch(const Pcg3dSeqPlan &plan, cudaStream_t stream) {
+    if (plan.rows) return pcg3d_rows_launch(*plan.rows, plan.state, stream);
     if (plan.resident) return pcg3d_res_launch(*plan.resident, plan.state, stream);
     if (plan.host_iterations > 0) return pcg3d_seq_run_host(plan, stream);
     return cudaGraphLaunch(plan.exec, stream);
@@ -1898,6 +1909,10 @@ cudaError_t pcg3d_seq_run_host(const Pcg3dSeqPlan &plan, cudaStream_t st) {
 }
 
 void pcg3d_seq_destroy(Pcg3dSeqPlan &plan) {
+    if (plan.rows) {
+        pcg3d_rows_destroy(*plan.rows);
+        delete plan.rows;
+    }
     if (plan.resident) {
         pcg3d_res_destroy(*plan.resident);
         delete plan.resident;

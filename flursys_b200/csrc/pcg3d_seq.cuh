@@ -23,8 +23,10 @@ struct CgSeqState {
 };
 
 struct Pcg3dResPlan;
+struct Pcg3dRowsPlan;
 
 struct Pcg3dSeqPlan {
+    Pcg3dRowsPlan *rows = nullptr;     // the chip-resident solve by rows, where it fits
     Pcg3dResPlan *resident = nullptr;  // the chip-resident solve replaces the graph when it fits
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
