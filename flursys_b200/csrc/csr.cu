@@ -13,12 +13,14 @@
 // direction update d = z + beta d is fused into the next SpMV: each gathered
 // column forms z[col] + beta d_old[col] on the fly (bit-identical wherever it
 // is formed) and the pass writes d_new for its own rows into a double buffer.
+// CG and PCG of matrices whose band fits the chip run in csr_band.cu instead.
 // BiCGSTAB follows bicgstab (solver.rs:155-256) with its early exit on ||s||.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -26,6 +28,7 @@
 #include "capi_internal.cuh"
 #include "common.cuh"
 #include "csr.cuh"
+#include "csr_band.cuh"
 
 namespace flursys {
 
@@ -387,6 +390,26 @@ struct DeviceCsr {
     }
 };
 
+// FLURSYS_CSR_BAND=0 keeps the kernel that streams its vectors.
+bool csr_band_enabled() {
+    const char *env = std::getenv("FLURSYS_CSR_BAND");
+    return !(env && std::strcmp(env, "0") == 0);
+}
+BandArgs band_args(const KrylovArgs &k, RedRecord *records, unsigned epoch) {
+    BandArgs a{};
+    a.n = k.a.n;
+    a.ro = k.a.ro; a.ci = k.a.ci; a.va = k.a.va;
+    a.inv_diag = k.method == 1 ? k.a.inv_diag : nullptr;
+    a.b = k.b;
+    a.x = k.x;
+    a.records = records;
+    a.epoch = epoch;
+    a.res = k.res;
+    a.atol = k.atol; a.rtol = k.rtol;
+    a.max_iters = k.max_iters;
+    return a;
+}
+
 int32_t csr_solve(int method, int64_t n, int64_t nnz, const int64_t *ro, const int64_t *ci, const double *va,
                   const double *rhs, double *x, const FlursysLinearSolverOptions *opt, FlursysLinearSolveReport *rep) {
     std::string msg;
@@ -441,9 +464,19 @@ int32_t csr_solve(int method, int64_t n, int64_t nnz, const int64_t *ro, const i
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, krylov_kernel, kBlock, 0);
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * per_sm, (n + kBlock * 4 - 1) / (kBlock * 4)));
+    BandPlan band;
+    if (method != 2 && csr_band_enabled()) {
+        int64_t reach = 0, width = 0;
+        for (int64_t r = 0; r < n; ++r) {
+            width = std::max(width, ro[r + 1] - ro[r]);
+            if (ro[r + 1] > ro[r]) reach = std::max({reach, r - ci[ro[r]], ci[ro[r + 1] - 1] - r});
+        }
+        band = csr_band_plan(n, reach, width, device);
+    }
     cudaStream_t stream;
     if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) return FLURSYS_ERR_CUDA;
     DeviceCsr A;
+    RedRecord *records = nullptr;
     std::vector<double *> bufs;
     auto alloc = [&](double **p, size_t cnt, cudaError_t *e) {
         if (*e == cudaSuccess) *e = cudaMalloc(p, sizeof(double) * std::max<size_t>(cnt, 1));
@@ -453,7 +486,7 @@ int32_t csr_solve(int method, int64_t n, int64_t nnz, const int64_t *ro, const i
     cudaError_t e = A.upload(n, nnz, ro, ci, va, stream);
     double *dinv = nullptr, *db = nullptr, *dx = nullptr;
     alloc(&db, n, &e); alloc(&dx, n, &e);
-    alloc(&k.r, n, &e); alloc(&k.z, n, &e); alloc(&k.d0, n, &e); alloc(&k.d1, n, &e); alloc(&k.q, n, &e);
+    if (band.blocks == 0) { alloc(&k.r, n, &e); alloc(&k.z, n, &e); alloc(&k.d0, n, &e); alloc(&k.d1, n, &e); alloc(&k.q, n, &e); }
     if (method == 2) { alloc(&k.rh, n, &e); alloc(&k.p, n, &e); alloc(&k.v, n, &e); alloc(&k.s, n, &e); alloc(&k.t, n, &e); }
     if (method == 1) alloc(&dinv, n, &e);
     alloc(&k.partials, (size_t)grid * kParts, &e);
@@ -479,7 +512,13 @@ int32_t csr_solve(int method, int64_t n, int64_t nnz, const int64_t *ro, const i
         k.max_iters = opt->max_iterations;
         k.method = method;
         void *params[] = {&k};
-        e = cudaLaunchCooperativeKernel((const void *)krylov_kernel, dim3(grid), dim3(kBlock), params, 0, stream);
+        if (band.blocks > 0) {
+            alloc(reinterpret_cast<double **>(&records), csr_band_record_bytes(band, n) / sizeof(double), &e);
+            if (e == cudaSuccess) e = cudaMemsetAsync(records, 0, csr_band_record_bytes(band, n), stream);
+            if (e == cudaSuccess) e = csr_band_launch(band, band_args(k, records, 1), stream);
+        } else {
+            e = cudaLaunchCooperativeKernel((const void *)krylov_kernel, dim3(grid), dim3(kBlock), params, 0, stream);
+        }
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(hres, dres, sizeof(CsrResultDev), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(x, dx, sizeof(double) * n, cudaMemcpyDeviceToHost, stream);
@@ -552,7 +591,22 @@ cudaError_t CsrDeviceWork::ensure(int n_, int device) {
     return e;
 }
 
+cudaError_t CsrDeviceWork::ensure_band(int n_, long long reach, long long width, int device, cudaStream_t st) {
+    if (!csr_band_enabled()) return cudaSuccess;
+    cudaFree(records);
+    records = nullptr;
+    band = csr_band_plan(n_, reach, width, device);
+    if (band.blocks == 0) return cudaSuccess;
+    cudaError_t e = cudaMalloc(&records, csr_band_record_bytes(band, n_));
+    if (e == cudaSuccess) e = cudaMemsetAsync(records, 0, csr_band_record_bytes(band, n_), st);
+    if (e != cudaSuccess) band = BandPlan{};
+    return e;
+}
+
 void CsrDeviceWork::release() {
+    cudaFree(records);
+    records = nullptr;
+    band = BandPlan{};
     cudaFree(vec); cudaFree(partials); cudaFree(inv_diag); cudaFree(bar); cudaFree(res);
     if (hres) cudaFreeHost(hres);
     vec = partials = inv_diag = nullptr;
@@ -588,7 +642,9 @@ cudaError_t csr_device_launch(int method, int n, const int *ro, const int *ci, c
     }
     if (e == cudaSuccess) {
         void *params[] = {&k};
-        e = cudaLaunchCooperativeKernel((const void *)krylov_kernel, dim3(w.grid), dim3(kBlock), params, 0, st);
+        e = method != 2 && w.band.blocks > 0
+                ? csr_band_launch(w.band, band_args(k, w.records, ++w.epoch), st)
+                : cudaLaunchCooperativeKernel((const void *)krylov_kernel, dim3(w.grid), dim3(kBlock), params, 0, st);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(w.hres, w.res, 2 * sizeof(CsrResultDev), cudaMemcpyDeviceToHost, st);
     return e;

@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "flursys_cuda.h"
+#include "gridreduce.cuh"
 
 namespace flursys {
 
@@ -21,6 +22,13 @@ struct CsrResultDev {
     unsigned pad;
 };
 
+// The split of a banded matrix over the chip (csr_band.cu).
+struct BandPlan {
+    int blocks = 0, rows = 0, band = 0, width = 0;  // blocks 0: the matrix does not fit
+    size_t smem = 0;
+    const void *kernel = nullptr;
+};
+
 // Work vectors of device-resident CSR solves (grown on demand), for callers
 // inside the library that assemble their matrices on the device.
 struct CsrDeviceWork {
@@ -31,7 +39,13 @@ struct CsrDeviceWork {
     GridBarrier *bar = nullptr;
     CsrResultDev *res = nullptr;   // [0] the solve, [1] the Jacobi set-up (error only)
     CsrResultDev *hres = nullptr;  // pinned copy of both
+    BandPlan band;                 // CG and PCG of a banded matrix
+    RedRecord *records = nullptr;  // its partial sums
+    unsigned epoch = 0;
     cudaError_t ensure(int n, int device);
+    // Lets CG and PCG solves of matrices with at most `width` entries in a row,
+    // all within `band` columns of the diagonal, run on the chip where they fit.
+    cudaError_t ensure_band(int n, long long band, long long width, int device, cudaStream_t st);
     void release();
 };
 

@@ -392,6 +392,7 @@ int32_t simple_channel_device(const FlursysSimpleConfig &c, double *hu, double *
     if (e == cudaSuccess) e = wu.ensure(n, device);
     if (e == cudaSuccess) e = wv.ensure(n, device);
     if (e == cudaSuccess) e = wp.ensure(n, device);
+    if (e == cudaSuccess) e = wp.ensure_band(n, nx, 5, device, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_ro, ro.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_ci, ci.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, st);
     // initial_face_flux: zero initial velocity; the inlet's prescribed flux
