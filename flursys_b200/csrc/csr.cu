@@ -581,12 +581,15 @@ cudaError_t CsrDeviceWork::ensure(int n_, int device) {
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, krylov_kernel, kBlock, 0);
     if (e != cudaSuccess) return e;
     grid = (int)std::max<long long>(1, std::min<long long>((long long)sms * per_sm, ((long long)n_ + kBlock * 4 - 1) / (kBlock * 4)));
-    e = cudaMalloc(&vec, sizeof(double) * 10 * (size_t)std::max(n_, 1));
-    if (e == cudaSuccess) e = cudaMalloc(&partials, sizeof(double) * kParts * (size_t)grid);
-    if (e == cudaSuccess) e = cudaMalloc(&inv_diag, sizeof(double) * (size_t)std::max(n_, 1));
-    if (e == cudaSuccess) e = cudaMalloc(&bar, sizeof(GridBarrier));
-    if (e == cudaSuccess) e = cudaMalloc(&res, 2 * sizeof(CsrResultDev));   // [0] solve, [1] Jacobi set-up
-    if (e == cudaSuccess) e = cudaMallocHost(&hres, 2 * sizeof(CsrResultDev));
+    const size_t rows = (size_t)std::max(n_, 1), parts = kParts * (size_t)grid;
+    e = cudaMalloc(&vec, sizeof(double) * (11 * rows + parts) + sizeof(GridBarrier) + 16 + 2 * sizeof(CsrResultDev));
+    if (e == cudaSuccess) {
+        inv_diag = vec + 10 * rows;
+        partials = inv_diag + rows;
+        bar = reinterpret_cast<GridBarrier *>(partials + parts);
+        res = reinterpret_cast<CsrResultDev *>(reinterpret_cast<char *>(bar) + (sizeof(GridBarrier) + 15) / 16 * 16);
+        e = cudaMallocHost(&hres, kCsrSlots * 2 * sizeof(CsrResultDev));
+    }
     if (e == cudaSuccess) n = n_;
     return e;
 }
@@ -599,15 +602,20 @@ cudaError_t CsrDeviceWork::ensure_band(int n_, long long reach, long long width,
     if (band.blocks == 0) return cudaSuccess;
     cudaError_t e = cudaMalloc(&records, csr_band_record_bytes(band, n_));
     if (e == cudaSuccess) e = cudaMemsetAsync(records, 0, csr_band_record_bytes(band, n_), st);
-    if (e != cudaSuccess) band = BandPlan{};
-    return e;
+    if (e != cudaSuccess) {  // no room: the streaming kernel serves every method
+        cudaGetLastError();
+        cudaFree(records);
+        records = nullptr;
+        band = BandPlan{};
+    }
+    return cudaSuccess;
 }
 
 void CsrDeviceWork::release() {
     cudaFree(records);
     records = nullptr;
     band = BandPlan{};
-    cudaFree(vec); cudaFree(partials); cudaFree(inv_diag); cudaFree(bar); cudaFree(res);
+    cudaFree(vec);
     if (hres) cudaFreeHost(hres);
     vec = partials = inv_diag = nullptr;
     bar = nullptr;
@@ -616,7 +624,7 @@ void CsrDeviceWork::release() {
 }
 
 cudaError_t csr_device_launch(int method, int n, const int *ro, const int *ci, const double *va, const double *b,
-                              double *x, double atol, double rtol, long long max_iters, CsrDeviceWork &w,
+                              double *x, double atol, double rtol, long long max_iters, CsrDeviceWork &w, int slot,
                               cudaStream_t st) {
     KrylovArgs k{};
     double *v = w.vec;
@@ -646,7 +654,7 @@ cudaError_t csr_device_launch(int method, int n, const int *ro, const int *ci, c
                 ? csr_band_launch(w.band, band_args(k, w.records, ++w.epoch), st)
                 : cudaLaunchCooperativeKernel((const void *)krylov_kernel, dim3(w.grid), dim3(kBlock), params, 0, st);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(w.hres, w.res, 2 * sizeof(CsrResultDev), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(w.hres + 2 * slot, w.res, 2 * sizeof(CsrResultDev), cudaMemcpyDeviceToHost, st);
     return e;
 }
 

@@ -29,16 +29,18 @@ struct BandPlan {
     const void *kernel = nullptr;
 };
 
+constexpr int kCsrSlots = 3;  // solves whose results a work area holds at a time
+
 // Work vectors of device-resident CSR solves (grown on demand), for callers
 // inside the library that assemble their matrices on the device.
 struct CsrDeviceWork {
     int n = 0, grid = 0;
-    double *vec = nullptr;       // 10 vectors of n
-    double *partials = nullptr;  // grid * 4
+    double *vec = nullptr;       // 10 vectors of n; the others follow in its allocation
     double *inv_diag = nullptr;  // n (PCG)
+    double *partials = nullptr;  // grid * 4
     GridBarrier *bar = nullptr;
     CsrResultDev *res = nullptr;   // [0] the solve, [1] the Jacobi set-up (error only)
-    CsrResultDev *hres = nullptr;  // pinned copy of both
+    CsrResultDev *hres = nullptr;  // pinned copies of both, by the launch's slot
     BandPlan band;                 // CG and PCG of a banded matrix
     RedRecord *records = nullptr;  // its partial sums
     unsigned epoch = 0;
@@ -52,12 +54,13 @@ struct CsrDeviceWork {
 // Enqueues one solve on device-resident CSR arrays (32-bit indices, columns
 // ascending in each row): method 0 CG, 1 Jacobi-PCG (the inverse diagonal is
 // formed on the device; a missing or zero diagonal is reported as an error),
-// 2 BiCGSTAB, with the stop rule of src/linear. The result record lands in
-// w.hres after the stream is synchronised; csr_device_status maps it.
+// 2 BiCGSTAB, with the stop rule of src/linear. The result records land in
+// w.hres + 2 * slot (slot < kCsrSlots) after the stream is synchronised;
+// csr_device_status maps them.
 // (b and x are not checked for finiteness beforehand: a non-finite value
 // surfaces as FLURSYS_ERR_NON_FINITE from the first SpMV or dot.)
 cudaError_t csr_device_launch(int method, int n, const int *ro, const int *ci, const double *va, const double *b,
-                              double *x, double atol, double rtol, long long max_iters, CsrDeviceWork &w,
+                              double *x, double atol, double rtol, long long max_iters, CsrDeviceWork &w, int slot,
                               cudaStream_t st);
 int32_t csr_device_status(const CsrResultDev *hres, FlursysLinearSolveReport *rep, std::string *err);
 

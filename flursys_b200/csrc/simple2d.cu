@@ -311,6 +311,23 @@ __global__ void __launch_bounds__(kBlk) k_continuity(Chan g, const double *__res
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
+// The 5-point pattern, columns ascending.
+__global__ void __launch_bounds__(kBlk) k_pattern(int nx, int ny, int *ro, int *ci) {
+    const int n = nx * ny;
+    for (int c = blockIdx.x * kBlk + threadIdx.x; c < n; c += gridDim.x * kBlk) {
+        const int j = c / nx, i = c - j * nx;
+        // entries of the rows of cells below, then of the cells before this one
+        int e = j * (5 * nx - 2) - (j > 0 ? nx : 0) + i * (5 - (j == 0) - (j == ny - 1)) - (i > 0);
+        ro[c] = e;
+        if (j > 0) ci[e++] = c - nx;
+        if (i > 0) ci[e++] = c - 1;
+        ci[e++] = c;
+        if (i + 1 < nx) ci[e++] = c + 1;
+        if (j + 1 < ny) ci[e++] = c + nx;
+        if (c == n - 1) ro[n] = e;
+    }
+}
+
 int grid_for(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + kBlk - 1) / kBlk, 148 * 8)); }
 
 int32_t fail(std::string *err, const std::string &msg, int32_t code) {
@@ -341,70 +358,61 @@ int32_t simple_channel_device(const FlursysSimpleConfig &c, double *hu, double *
         return fail(err, "continuity tolerance must be finite and non-negative", FLURSYS_ERR_INVALID_CONFIG);
     const int nx = (int)c.nx, ny = (int)c.ny, n = nx * ny;
     const int nfx = (nx + 1) * ny, nfy = nx * (ny + 1);
-    // 5-point pattern
-    std::vector<int> ro(n + 1), ci;
-    ci.reserve((size_t)n * 5);
-    for (int j = 0; j < ny; ++j)
-        for (int i = 0; i < nx; ++i) {
-            const int cc = i + nx * j;
-            ro[cc] = (int)ci.size();
-            if (j > 0) ci.push_back(cc - nx);
-            if (i > 0) ci.push_back(cc - 1);
-            ci.push_back(cc);
-            if (i + 1 < nx) ci.push_back(cc + 1);
-            if (j + 1 < ny) ci.push_back(cc + nx);
-        }
-    ro[n] = (int)ci.size();
-    const int nnz = ro[n];
+    const int nnz = 5 * n - 2 * nx - 2 * ny;  // 5-point pattern
     int device = 0;
     cudaGetDevice(&device);
     cudaStream_t st;
     cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e != cudaSuccess) return set_cuda_error(err, e, "SIMPLE stream");
-    std::vector<void *> allocs;
-    auto dalloc = [&](size_t bytes) -> void * {
-        void *q = nullptr;
-        if (e == cudaSuccess) e = cudaMalloc(&q, std::max<size_t>(bytes, 8));
-        if (e == cudaSuccess) {
-            allocs.push_back(q);
-            e = cudaMemsetAsync(q, 0, std::max<size_t>(bytes, 8), st);
-        }
+    // One device allocation for the fields and one pinned one for the scalars
+    // that come back: separate ones cost more than the assembly kernels.
+    const int ncb = grid_for(n);
+    char *slab = nullptr;
+    size_t slab_bytes = 0;
+    auto carve = [&](size_t bytes) -> char * {
+        char *q = slab ? slab + slab_bytes : nullptr;
+        slab_bytes += (std::max<size_t>(bytes, 8) + 255) / 256 * 256;
         return q;
     };
-    int *d_ro = (int *)dalloc(sizeof(int) * (n + 1));
-    int *d_ci = (int *)dalloc(sizeof(int) * nnz);
-    double *mvals = (double *)dalloc(8.0 * nnz), *pvals = (double *)dalloc(8.0 * nnz);
-    double *u = (double *)dalloc(8.0 * n), *v = (double *)dalloc(8.0 * n), *p = (double *)dalloc(8.0 * n);
-    double *us = (double *)dalloc(8.0 * n), *vs = (double *)dalloc(8.0 * n), *pc = (double *)dalloc(8.0 * n);
-    double *gx = (double *)dalloc(8.0 * n), *gy = (double *)dalloc(8.0 * n), *rau = (double *)dalloc(8.0 * n);
-    double *bu = (double *)dalloc(8.0 * n), *bv = (double *)dalloc(8.0 * n), *prhs = (double *)dalloc(8.0 * n);
-    double *Fx = (double *)dalloc(8.0 * nfx), *Fy = (double *)dalloc(8.0 * nfy);
-    double *Fxp = (double *)dalloc(8.0 * nfx), *Fyp = (double *)dalloc(8.0 * nfy);
-    double *cfx = (double *)dalloc(8.0 * nfx), *cfy = (double *)dalloc(8.0 * nfy);
-    const int ncb = grid_for(n);
-    double *part = (double *)dalloc(8.0 * ncb);
-    int *flag = (int *)dalloc(sizeof(int));
+    int *d_ro, *d_ci, *flag;
+    double *mvals, *pvals, *u, *v, *p, *us, *vs, *pc, *gx, *gy, *rau, *bu, *bv, *prhs, *Fx, *Fy, *Fxp, *Fyp, *cfx, *cfy, *part;
+    auto lay_out = [&]() {
+        slab_bytes = 0;
+        d_ro = (int *)carve(sizeof(int) * (n + 1));
+        d_ci = (int *)carve(sizeof(int) * nnz);
+        flag = (int *)carve(sizeof(int));
+        for (double **q : {&mvals, &pvals}) *q = (double *)carve(8.0 * nnz);
+        for (double **q : {&u, &v, &p, &us, &vs, &pc, &gx, &gy, &rau, &bu, &bv, &prhs}) *q = (double *)carve(8.0 * n);
+        for (double **q : {&Fx, &Fxp, &cfx}) *q = (double *)carve(8.0 * nfx);
+        for (double **q : {&Fy, &Fyp, &cfy}) *q = (double *)carve(8.0 * nfy);
+        part = (double *)carve(8.0 * ncb);
+    };
+    lay_out();
+    e = cudaMalloc(&slab, slab_bytes);
+    if (e == cudaSuccess) lay_out();
+    if (e == cudaSuccess) e = cudaMemsetAsync(slab, 0, slab_bytes, st);
     double *h_part = nullptr;
-    int *h_flag = nullptr;
-    if (e == cudaSuccess) e = cudaMallocHost(&h_part, 8 * ncb);
-    if (e == cudaSuccess) e = cudaMallocHost(&h_flag, sizeof(int));
-    CsrDeviceWork wu, wv, wp;
-    if (e == cudaSuccess) e = wu.ensure(n, device);
-    if (e == cudaSuccess) e = wv.ensure(n, device);
-    if (e == cudaSuccess) e = wp.ensure(n, device);
-    if (e == cudaSuccess) e = wp.ensure_band(n, nx, 5, device, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_ro, ro.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_ci, ci.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMallocHost(&h_part, 8 * (ncb + ny + 1));
+    int *h_flag = reinterpret_cast<int *>(h_part + ncb);
+    CsrDeviceWork work;  // of the three solves, one after another
+    if (e == cudaSuccess) e = work.ensure(n, device);
+    if (e == cudaSuccess) e = work.ensure_band(n, nx, 5, device, st);
+    if (e == cudaSuccess) {
+        k_pattern<<<ncb, kBlk, 0, st>>>(nx, ny, d_ro, d_ci);
+        e = cudaGetLastError();
+    }
     // initial_face_flux: zero initial velocity; the inlet's prescribed flux
     // (owner-oriented u_in * (-dy), i.e. +x flux u_in * dy); walls 0.
-    std::vector<double> fx0(nfx, 0.0);
     const double dx = c.length / nx, dy = c.height / ny;
-    for (int j = 0; j < ny; ++j) {
-        const double y = (j + 0.5) * dy;
-        const double uin = c.inlet_peak_velocity * 4.0 * y * (c.height - y) / (c.height * c.height);
-        fx0[(nx + 1) * j] = -(uin * (-dy));
+    if (e == cudaSuccess) {
+        double *fx0 = h_part + ncb + 1;
+        for (int j = 0; j < ny; ++j) {
+            const double y = (j + 0.5) * dy;
+            const double uin = c.inlet_peak_velocity * 4.0 * y * (c.height - y) / (c.height * c.height);
+            fx0[j] = -(uin * (-dy));
+        }
+        e = cudaMemcpy2DAsync(Fx, 8.0 * (nx + 1), fx0, 8, 8, ny, cudaMemcpyHostToDevice, st);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(Fx, fx0.data(), 8 * nfx, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     int32_t status = FLURSYS_OK;
     std::vector<double> hist;
@@ -442,16 +450,16 @@ int32_t simple_channel_device(const FlursysSimpleConfig &c, double *hu, double *
         if (e == cudaSuccess) e = cudaMemcpyAsync(vs, v, 8.0 * n, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess)
             e = csr_device_launch(2, n, d_ro, d_ci, mvals, bu, us, mo.absolute_tolerance, mo.relative_tolerance,
-                                  mo.max_iterations, wu, st);
+                                  mo.max_iterations, work, 0, st);
         if (e == cudaSuccess)
             e = csr_device_launch(2, n, d_ro, d_ci, mvals, bv, vs, mo.absolute_tolerance, mo.relative_tolerance,
-                                  mo.max_iterations, wv, st);
+                                  mo.max_iterations, work, 1, st);
         k_rhie_chow<<<nfb, kBlk, 0, st>>>(g, us, vs, p, gx, gy, rau, Fx, Fy, Fxp, Fyp, cfx, cfy);
         k_passemble<<<ncb, kBlk, 0, st>>>(g, Fxp, Fyp, cfx, cfy, pvals, prhs);
         if (e == cudaSuccess) e = cudaMemsetAsync(pc, 0, 8.0 * n, st);
         if (e == cudaSuccess)
             e = csr_device_launch(1, n, d_ro, d_ci, pvals, prhs, pc, po.absolute_tolerance, po.relative_tolerance,
-                                  po.max_iterations, wp, st);
+                                  po.max_iterations, work, 2, st);
         k_grad<<<ncb, kBlk, 0, st>>>(g, pc, c.outlet_pressure, gx, gy);
         k_velocity<<<ncb, kBlk, 0, st>>>(n, c.pressure_relaxation, pc, p, us, vs, rau, gx, gy, u, v);
         k_flux<<<nfb, kBlk, 0, st>>>(g, Fxp, Fyp, cfx, cfy, pc, Fx, Fy);
@@ -462,9 +470,9 @@ int32_t simple_channel_device(const FlursysSimpleConfig &c, double *hu, double *
         if (e != cudaSuccess) { status = set_cuda_error(err, e, "SIMPLE outer iteration"); break; }
         if (*h_flag & 1) { status = fail(err, "backflow on a zero-gradient velocity boundary face", FLURSYS_ERR_INVALID_CONFIG); break; }
         if (*h_flag & 2) { status = fail(err, "invalid momentum diagonal", FLURSYS_ERR_BREAKDOWN); break; }
-        if ((status = csr_device_status(wu.hres, &rep->momentum[0], err))) break;
-        if ((status = csr_device_status(wv.hres, &rep->momentum[1], err))) break;
-        if ((status = csr_device_status(wp.hres, &rep->pressure, err))) break;
+        if ((status = csr_device_status(work.hres + 2 * 0, &rep->momentum[0], err))) break;
+        if ((status = csr_device_status(work.hres + 2 * 1, &rep->momentum[1], err))) break;
+        if ((status = csr_device_status(work.hres + 2 * 2, &rep->pressure, err))) break;
         rep->momentum[2] = FlursysLinearSolveReport{FLURSYS_LINEAR_CONVERGED, 0, 0, 0.0, 0.0, 0.0};
         if (rep->momentum[0].status != FLURSYS_LINEAR_CONVERGED || rep->momentum[1].status != FLURSYS_LINEAR_CONVERGED) {
             status = fail(err, "momentum linear solve did not converge", FLURSYS_ERR_BREAKDOWN);
@@ -488,9 +496,10 @@ int32_t simple_channel_device(const FlursysSimpleConfig &c, double *hu, double *
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
         rep->solve_ms = ms;
-        std::vector<double> hfx(nfx), hfy(nfy);
-        e = cudaMemcpyAsync(hfx.data(), Fx, 8 * nfx, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hfy.data(), Fy, 8 * nfy, cudaMemcpyDeviceToHost, st);
+        std::vector<double> own_flux(hflux ? 0 : (size_t)nfx + nfy);
+        double *hfx = hflux ? hflux : own_flux.data(), *hfy = hfx + nfx;
+        e = cudaMemcpyAsync(hfx, Fx, 8.0 * nfx, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(hfy, Fy, 8.0 * nfy, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess && hu) e = cudaMemcpyAsync(hu, u, 8.0 * n, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess && hv) e = cudaMemcpyAsync(hv, v, 8.0 * n, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess && hp) e = cudaMemcpyAsync(hp, p, 8.0 * n, cudaMemcpyDeviceToHost, st);
@@ -510,21 +519,14 @@ int32_t simple_channel_device(const FlursysSimpleConfig &c, double *hu, double *
             for (int j = 0; j < ny; ++j) acc(hfx[nx + (nx + 1) * j]);
             for (int i = 0; i < nx; ++i) acc(-hfy[i]);
             for (int i = 0; i < nx; ++i) acc(hfy[i + nx * ny]);
-            if (hflux) {
-                std::memcpy(hflux, hfx.data(), 8 * nfx);
-                std::memcpy(hflux + nfx, hfy.data(), 8 * nfy);
-            }
             if (hhist) std::memcpy(hhist, hist.data(), 8 * hist.size());
         }
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    wu.release();
-    wv.release();
-    wp.release();
-    for (void *q : allocs) cudaFree(q);
+    work.release();
+    cudaFree(slab);
     if (h_part) cudaFreeHost(h_part);
-    if (h_flag) cudaFreeHost(h_flag);
     cudaStreamDestroy(st);
     return status;
 }
