@@ -902,6 +902,7 @@ cudaError_t pcg2d_res_plan(Pcg2dResPlan &plan, int nx, int ny, bool plain, int p
     }
     e = cudaMalloc(&plan.records, bytes);
     if (e == cudaSuccess) e = cudaMemset(plan.records, 0, bytes);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // solves run on streams that do not wait for this one
     plan.enabled = e == cudaSuccess;
     return e;
 }

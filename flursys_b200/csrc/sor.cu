@@ -391,6 +391,7 @@ cudaError_t sor3d_plan(Sor3dPlan &plan, int nx, int ny, int nz, int device) {
     const size_t bytes = sizeof(RedRecord) * 2 * ng * (kRedSlots + 2 * (size_t)half_row(nx) * ny);
     e = cudaMalloc(&plan.records, bytes);
     if (e == cudaSuccess) e = cudaMemset(plan.records, 0, bytes);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // solves run on streams that do not wait for this one
     if (e == cudaSuccess) plan.blocks = ng;
     return e;
 }
