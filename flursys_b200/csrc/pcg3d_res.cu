@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(BLK, 1) pcg3d_res1_kernel(const __grid_constan
 bool pcg3d_res_plan(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device) {
     plan = Pcg3dResPlan{};
     const char *env = std::getenv("FLURSYS_PCG_RESIDENT");
-    if (env && std::strcmp(env, "0") == 0) return false;
+    if (env && (std::strcmp(env, "0") == 0 || std::strcmp(env, "stream") == 0)) return false;
     if (args.nz < 2) return false;
     ResArgs &a = plan.args;
     a.nx = args.nx; a.ny = args.ny; a.nz = args.nz;

@@ -49,7 +49,7 @@ struct Pcg3dResPlan {
 
 // Sets up the resident solve for `args` (MIXED work vectors: args.r and
 // args.q are the FP32 face-exchange buffers); false when the grid does not fit one tile per
-// SM, the device cannot hold a tile, or FLURSYS_PCG_RESIDENT=0.
+// SM, the device cannot hold a tile, or FLURSYS_PCG_RESIDENT asks for another form.
 bool pcg3d_res_plan(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device);
 // One solve; the result is written to *state (CgSeqState fields error,
 // status, iterations, initial, initial_l2, residual, true_l2, device_error).

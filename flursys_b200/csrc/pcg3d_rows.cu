@@ -749,9 +749,10 @@ bool choose_rows(Pcg3dRowsPlan &plan, int sms, bool may_cluster, bool may_grid) 
 
 bool pcg3d_rows_plan(Pcg3dRowsPlan &plan, const Pcg3dArgs &args, int precision, int device) {
     plan = Pcg3dRowsPlan{};
-    // FLURSYS_PCG_RESIDENT: 0 and 2 ask for other forms, "grid" for no cluster
+    // FLURSYS_PCG_RESIDENT: 0, 2 and "stream" ask for other forms, "grid" for
+    // no cluster
     const char *env = std::getenv("FLURSYS_PCG_RESIDENT");
-    if (env && (std::strcmp(env, "0") == 0 || std::strcmp(env, "2") == 0)) return false;
+    if (env && (std::strcmp(env, "0") == 0 || std::strcmp(env, "2") == 0 || std::strcmp(env, "stream") == 0)) return false;
     if (args.nz < 2) return false;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return false;
@@ -797,7 +798,9 @@ bool pcg3d_rows_plan(Pcg3dRowsPlan &plan, const Pcg3dArgs &args, int precision, 
     if (!plan.cluster) {
         const size_t rec = sizeof(RedRecord) * 2 * plan.blocks * kRedSlots;
         const size_t slots = mixed ? face_values<float>(a.nx, a.ty, a.tz) : face_values<double>(a.nx, a.ty, a.tz);
+        // (the clearing ends here: solves run on streams that do not wait for this one)
         if (cudaMalloc(&plan.records, rec) != cudaSuccess || cudaMemset(plan.records, 0, rec) != cudaSuccess ||
+            cudaStreamSynchronize(nullptr) != cudaSuccess ||
             cudaMalloc(&plan.faces, (mixed ? 4 : 8) * 2 * plan.blocks * slots) != cudaSuccess) {
             pcg3d_rows_destroy(plan);
             return false;

@@ -35,6 +35,7 @@
 #include "pcg3d_seq.cuh"
 #include "pcg3d_res.cuh"
 #include "pcg3d_rows.cuh"
+#include "pcg3d_stream.cuh"
 #include "tma.cuh"
 
 namespace flursys {
@@ -1791,6 +1792,36 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
     // (instruction-bound by the halo recomputation, 238 instructions per cell).
     const char *cg1_env = std::getenv("FLURSYS_PCG_CG1");
     a.cg1 = precision == FLURSYS_PRECISION_MIXED && g.nx % 4 == 0 && cg1_env && std::strcmp(cg1_env, "1") == 0;
+    const char *v = std::getenv("FLURSYS_PCG_VARIANT");
+    if (v && std::strcmp(v, "host") == 0) plan.host_iterations = 1;
+    // Which form serves a grid (us per iteration):
+    // - F64 and MIXED grids whose rows fit the chip: pcg3d_rows.cu, less than
+    //   every other form at all sizes that it holds (128^3 MIXED 16 | tiles 20);
+    // - MIXED grids between that and one 32 x 32 x tz tile per SM: pcg3d_res.cu
+    //   (192 x 128 x 96: tiles 20.5 | streaming 21.2 | graph 34);
+    // - larger ones whose planes fit a block: pcg3d_stream.cu (160^3 MIXED 30 |
+    //   graph 50, 256^3 MIXED 103 | 139, 112^3 F64 22 | 43, 200^3 F64 124 | 184);
+    // - the rest (rows above about 700 cells): the graph.
+    // FLURSYS_PCG_RESIDENT=0 keeps the graph, =2 the tiles, =stream the
+    // streaming form.
+    if (!a.cg1 && plan.host_iterations == 0) {
+        auto *rp = new Pcg3dRowsPlan();
+        if (pcg3d_rows_plan(*rp, args, precision, device)) plan.rows = rp;
+        else delete rp;
+        cudaGetLastError();  // a declined plan leaves no sticky error behind
+    }
+    if (!plan.rows && precision == FLURSYS_PRECISION_MIXED && !a.cg1 && plan.host_iterations == 0) {
+        auto *rp = new Pcg3dResPlan();
+        if (pcg3d_res_plan(*rp, args, device)) plan.resident = rp;
+        else delete rp;
+        cudaGetLastError();  // a declined plan leaves no sticky error behind
+    }
+    if (!plan.rows && !plan.resident && !a.cg1 && plan.host_iterations == 0) {
+        auto *sp = new Pcg3dStreamPlan();
+        if (pcg3d_stream_plan(*sp, args, precision, device)) plan.stream = sp;
+        else delete sp;
+        cudaGetLastError();
+    }
     Cg1Maps maps{};
     if (a.cg1) {
         a.cr[0] = static_cast<float *>(args.r);
@@ -1814,34 +1845,16 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
         if (e != cudaSuccess) return e;
         plan.cg1_maps = new Cg1Maps(maps);
         e = build_cg1(plan, a, maps);
-    } else {
+    } else if (!plan.rows && !plan.resident && !plan.stream) {
         e = precision == FLURSYS_PRECISION_MIXED ? build<float, true>(plan, a) : build<double, false>(plan, a);
     }
     plan.host_args = new SeqArgs(a);
-    const char *v = std::getenv("FLURSYS_PCG_VARIANT");
-    if (v && std::strcmp(v, "host") == 0) plan.host_iterations = 1;
-    // Solves whose rows fit the chip run resident, one launch per solve, F64
-    // and MIXED (pcg3d_rows.cu: less per iteration than every other form at all
-    // sizes that it holds). MIXED grids between that and one 32 x 32 x tz tile
-    // per SM (192 x 128 x 96) keep the tile-resident form (pcg3d_res.cu).
-    // FLURSYS_PCG_RESIDENT=0 keeps the graph, =2 the tile-resident form.
-    if (e == cudaSuccess && !a.cg1 && plan.host_iterations == 0) {
-        auto *rp = new Pcg3dRowsPlan();
-        if (pcg3d_rows_plan(*rp, args, precision, device)) plan.rows = rp;
-        else delete rp;
-        cudaGetLastError();  // a declined plan leaves no sticky error behind
-    }
-    if (e == cudaSuccess && !plan.rows && precision == FLURSYS_PRECISION_MIXED && !a.cg1 && plan.host_iterations == 0) {
-        auto *rp = new Pcg3dResPlan();
-        if (pcg3d_res_plan(*rp, args, device)) plan.resident = rp;
-        else delete rp;
-        cudaGetLastError();  // a declined plan leaves no sticky error behind
-    }
     return e;
 }
 
 cudaError_t pcg3d_seq_launch(const Pcg3dSeqPlan &plan, cudaStream_t stream) {
     if (plan.rows) return pcg3d_rows_launch(*plan.rows, plan.state, stream);
+    if (plan.stream) return pcg3d_stream_launch(*plan.stream, plan.state, stream);
     if (plan.resident) return pcg3d_res_launch(*plan.resident, plan.state, stream);
     if (plan.host_iterations > 0) return pcg3d_seq_run_host(plan, stream);
     return cudaGraphLaunch(plan.exec, stream);
@@ -1912,6 +1925,10 @@ void pcg3d_seq_destroy(Pcg3dSeqPlan &plan) {
     if (plan.rows) {
         pcg3d_rows_destroy(*plan.rows);
         delete plan.rows;
+    }
+    if (plan.stream) {
+        pcg3d_stream_destroy(*plan.stream);
+        delete plan.stream;
     }
     if (plan.resident) {
         pcg3d_res_destroy(*plan.resident);

@@ -24,9 +24,11 @@ struct CgSeqState {
 
 struct Pcg3dResPlan;
 struct Pcg3dRowsPlan;
+struct Pcg3dStreamPlan;
 
 struct Pcg3dSeqPlan {
     Pcg3dRowsPlan *rows = nullptr;     // the chip-resident solve by rows, where it fits
+    Pcg3dStreamPlan *stream = nullptr; // the solve that streams its vectors once per iteration
     Pcg3dResPlan *resident = nullptr;  // the chip-resident solve replaces the graph when it fits
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
