@@ -1799,9 +1799,10 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
     //   every other form at all sizes that it holds (128^3 MIXED 16 | tiles 20);
     // - MIXED grids between that and one 32 x 32 x tz tile per SM: pcg3d_res.cu
     //   (192 x 128 x 96: tiles 20.5 | streaming 21.2 | graph 34);
-    // - larger ones whose planes fit a block: pcg3d_stream.cu (160^3 MIXED 30 |
-    //   graph 50, 256^3 MIXED 103 | 139, 112^3 F64 22 | 43, 200^3 F64 124 | 184);
-    // - the rest (rows above about 700 cells): the graph.
+    // - larger ones whose planes fit a block: pcg3d_stream.cu (150 x 120 x 130
+    //   MIXED 22 | graph 60, 112^3 F64 22 | 43, 200^3 F64 124 | 184), MIXED up
+    //   to 3.2 million cells (see there);
+    // - the rest (rows above about 700 cells, larger MIXED grids): the graph.
     // FLURSYS_PCG_RESIDENT=0 keeps the graph, =2 the tiles, =stream the
     // streaming form.
     if (!a.cg1 && plan.host_iterations == 0) {

@@ -297,12 +297,13 @@ int32_t flursys_cuda_set_stream(FlursysCudaHandle *h, void *stream);
 /* Device-time split of the last pressure solve of this handle, in ms:
  * [0] stencil passes, [1] pointwise passes, [2] grid barriers and partial
  * reductions, [3] FP64 residual replacements (as seen by block 0). For the
- * chip-resident 3D solve (FLURSYS_SOLVE_RESIDENT) the split is [0] face
- * exchange and direction update, [1] operator pass, [2] grid reductions and
- * barriers, [3] vector updates and residual replacements, [4] block 0's
- * waits inside grid barriers, [5] the largest [0] + [1] + [3] of any block
- * (the slowest block's work); the graph-driven 3D solve records none (all
- * zero). `n` is the capacity of `phase_ms` (up to 6 used). No reference
+ * chip-resident 3D solves (FLURSYS_SOLVE_RESIDENT) the split is [0] direction
+ * (and, by tiles, face exchange), [1] operator pass, [2] grid reductions and
+ * barriers, [3] residual replacements (by tiles also vector updates), [4]
+ * block 0's waits inside grid barriers (by tiles), [5] the largest [0] + [1] +
+ * [3] of any block (the slowest block's work); for the 3D solve that streams
+ * its vectors in one pass [1] is the passes, [2] and [3] as above; the
+ * graph-driven 3D solve records none (all zero). `n` is the capacity of `phase_ms` (up to 6 used). No reference
  * counterpart. */
 int32_t flursys_cuda_solver_profile(const FlursysCudaHandle *h, double *phase_ms, size_t n);
 
@@ -553,7 +554,7 @@ enum FlursysBatchFlags {
 typedef struct FlursysBatchTuning {
     int32_t tile_elems[6];      /* elements per tile: predict, boundaries, rhs, correct, boundaries, post */
     int32_t pressure_blocks_per_sm;
-    int32_t pressure_blocks;    /* blocks of the cooperative pressure launch */
+    int32_t pressure_blocks;    /* blocks of the pressure launch that streams its vectors */
     int32_t graph_nodes;        /* kernel nodes of one step's graph (0 without a graph) */
     int32_t reserved;
     double tune_ms;             /* host time spent tuning at create */
