@@ -166,14 +166,66 @@ __global__ void __launch_bounds__(kPw) fcg_shift(double *x, const FcgScalars *sc
 }
 
 // Smoothing passes of the preconditioner (damped Jacobi on A~, weight
-// omega; pre: z = omega D^-1 r and r - A~ z; post: z_in + omega D^-1
-// (r - A~ z_in)) and the operator pass, as z-marching FP32 stencil passes.
-// A block owns a 32 x kBY column of cells over kMZ planes; each thread keeps
-// the operand of the plane below, its own and the one above in registers,
-// so a plane is read from memory once per block (x and y neighbours come
-// through L1), and the block's partial sums are reduced once, after the
-// march. The operator arithmetic per cell is that of apply7, in its order.
-constexpr int kMZ = 16;  // planes per marching block
+// omega; pre: z0 = omega D^-1 r and r - A~ z0; post: z_in + omega D^-1
+// (r - A~ z_in) with z_in = z0 + z_net) and the operator pass, as z-marching
+// FP32 stencil passes. A thread owns four cells of x and marches `kz` planes:
+// the operand of the plane below, its own and the one above lie in registers,
+// x and y neighbours come through L1. z0 is formed again where it is needed
+// instead of stored. The operator arithmetic per cell is that of apply7, in
+// its order, with weight 0 where there is no neighbour.
+//
+// What bounds them: HBM (8, 12 and 12 bytes per cell; a thread per cell, with
+// its neighbour tests, was bound by issue). Per pass on 256^3, before and
+// after: operator 56 and 44 us, pre-smoothing 69 and 30, post-smoothing 73 and 44.
+struct March {
+    int nvec, kz;  // vectors of a row, planes of a block
+};
+struct Column {
+    int v, j;
+    bool in, first, last;  // inside the grid; first and last vector of a row
+    long long c, sy;       // cell at plane 0; row stride
+    float wym, wyp;
+};
+__device__ __forceinline__ Column march_column(const Geo3 &g, const March &m) {
+    const int t = blockIdx.x * (kBX * kBY) + threadIdx.x;
+    Column o;
+    o.j = t / m.nvec;
+    o.v = t - o.j * m.nvec;
+    o.in = o.j < g.ny;
+    if (!o.in) o.j = o.v = 0;
+    o.first = o.v == 0;
+    o.last = o.v == m.nvec - 1;
+    o.sy = g.nx;
+    o.c = (long long)o.j * g.nx + 4 * o.v;
+    o.wym = o.j > 0 ? g.wy : 0.f;
+    o.wyp = o.j + 1 < g.ny ? g.wy : 0.f;
+    return o;
+}
+__device__ __forceinline__ void ld4(const float *p, float (&v)[4]) {
+    const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void st4(float *p, const float (&v)[4]) {
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+// A~ of four cells; we, ea: the cells before and behind them.
+__device__ __forceinline__ void apply7x4(const Geo3 &g, const Column &o, float wzm, float wzp, const float (&c)[4], float we,
+                                         float ea, const float (&so)[4], const float (&no)[4], const float (&be)[4],
+                                         const float (&ab)[4], float (&out)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float wxm = e == 0 && o.first ? 0.f : g.wx, wxp = e == 3 && o.last ? 0.f : g.wx;
+        const float xw = e ? c[e ? e - 1 : 0] : we, xe = e < 3 ? c[e < 3 ? e + 1 : 3] : ea;
+        const float dg = ((((wxm + wxp) + o.wym) + o.wyp) + wzm) + wzp;
+        float s = wxm * xw;
+        s += wxp * xe;
+        s += o.wym * so[e];
+        s += o.wyp * no[e];
+        s += wzm * be[e];
+        s += wzp * ab[e];
+        out[e] = dg * c[e] - s;
+    }
+}
 
 // omega / diag of the Neumann-form operator by missing-neighbour class
 // 9 mx + 3 my + mz (FP32, formed in FP64 on the host), so the smoothing
@@ -182,80 +234,131 @@ struct SmoothW {
     float winv[27];
 };
 __device__ __forceinline__ int miss3(int i, int n) { return (i == 0) + (i == n - 1); }
-__device__ __forceinline__ float winv_at(const SmoothW &w, const Geo3 &g, int i, int j, int k) {
-    return w.winv[9 * miss3(i, g.nx) + 3 * miss3(j, g.ny) + miss3(k, g.nz)];
+// The weights of a column's four cells in a row of class yz = 3 my + mz, and
+// those of the cells before and behind them (never at a wall of x).
+__device__ __forceinline__ void winv4(const SmoothW &w, const Column &o, int yz, float (&m)[4]) {
+    const float mid = w.winv[yz], edge = w.winv[9 + yz];
+    m[0] = o.first ? edge : mid;
+    m[1] = m[2] = mid;
+    m[3] = o.last ? edge : mid;
 }
 
 // q = A~ d (Neumann form, FP32); partials d.q and d.r.
-__global__ void __launch_bounds__(kBX * kBY) fcg_spmv_m(Geo3 g, const float *__restrict__ d,
+__global__ void __launch_bounds__(kBX * kBY) fcg_spmv_m(Geo3 g, March m, const float *__restrict__ d,
                                                         const float *__restrict__ r, float *q, double *partials) {
-    const int i = blockIdx.x * kBX + (threadIdx.x & 31), j = blockIdx.y * kBY + (threadIdx.x >> 5);
-    const int k0 = blockIdx.z * kMZ, k1 = min(g.nz, k0 + kMZ);
+    const Column o = march_column(g, m);
+    const int k0 = blockIdx.y * m.kz, k1 = min(g.nz, k0 + m.kz);
     double v[2] = {0.0, 0.0};
-    if (i < g.nx && j < g.ny) {
-        const long long sy = g.nx, sz = (long long)g.nx * g.ny;
-        long long c = ((long long)k0 * g.ny + j) * g.nx + i;
-        float below = k0 > 0 ? d[c - sz] : 0.f, cur = d[c];
+    if (o.in) {
+        const long long sz = (long long)g.nx * g.ny;
+        long long c = o.c + k0 * sz;
+        float be[4], cu[4], ab[4], so[4], no[4], rv[4], qv[4];
+        ld4(d + c, cu);
+        ld4(d + (k0 > 0 ? c - sz : c), be);
         for (int k = k0; k < k1; ++k, c += sz) {
-            const float above = k + 1 < g.nz ? d[c + sz] : 0.f;
-            const float qv = apply7<float>(g, i, j, k, g.wx, g.wy, g.wz, cur, [&](int a, int b, int e) {
-                return e < 0 ? below : (e > 0 ? above : d[c + a + b * sy]);
-            });
-            q[c] = qv;
-            v[0] += double(cur) * double(qv);
-            v[1] += double(cur) * double(r[c]);
-            below = cur;
-            cur = above;
+            const bool up = k + 1 < g.nz;
+            ld4(d + (up ? c + sz : c), ab);
+            ld4(d + (o.j > 0 ? c - o.sy : c), so);
+            ld4(d + (o.j + 1 < g.ny ? c + o.sy : c), no);
+            ld4(r + c, rv);
+            const float we = o.first ? cu[0] : __ldg(d + c - 1), ea = o.last ? cu[3] : __ldg(d + c + 4);
+            apply7x4(g, o, k > 0 ? g.wz : 0.f, up ? g.wz : 0.f, cu, we, ea, so, no, be, ab, qv);
+            st4(q + c, qv);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                v[0] += double(cu[e]) * double(qv[e]);
+                v[1] += double(cu[e]) * double(rv[e]);
+                be[e] = cu[e];
+                cu[e] = ab[e];
+            }
         }
     }
-    const int blk = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    write_partials(partials, blk, v, 2);
+    write_partials(partials, blockIdx.y * gridDim.x + blockIdx.x, v, 2);
 }
 
-// Pre-smoothing: z_out = omega D^-1 r, r_out = r - A~ z_out.
-__global__ void __launch_bounds__(kBX * kBY) fcg_presmooth_m(Geo3 g, const float *__restrict__ r, float *z_out,
-                                                             float *r_out, const __grid_constant__ SmoothW w) {
-    const int i = blockIdx.x * kBX + (threadIdx.x & 31), j = blockIdx.y * kBY + (threadIdx.x >> 5);
-    const int k0 = blockIdx.z * kMZ, k1 = min(g.nz, k0 + kMZ);
-    if (i >= g.nx || j >= g.ny) return;
-    const long long sy = g.nx, sz = (long long)g.nx * g.ny;
-    long long c = ((long long)k0 * g.ny + j) * g.nx + i;
-    auto zat = [&](long long m, int ii, int jj, int kk) { return r[m] * winv_at(w, g, ii, jj, kk); };
-    float below = k0 > 0 ? zat(c - sz, i, j, k0 - 1) : 0.f, cur = zat(c, i, j, k0);
+// Pre-smoothing: r_out = r - A~ z0, z0 = omega D^-1 r.
+__global__ void __launch_bounds__(kBX * kBY) fcg_presmooth_m(Geo3 g, March m, const float *__restrict__ r, float *r_out,
+                                                             const __grid_constant__ SmoothW w) {
+    const Column o = march_column(g, m);
+    const int k0 = blockIdx.y * m.kz, k1 = min(g.nz, k0 + m.kz);
+    if (!o.in) return;
+    const long long sz = (long long)g.nx * g.ny;
+    long long c = o.c + k0 * sz;
+    const int yc = 3 * miss3(o.j, g.ny), ys = 3 * miss3(max(o.j - 1, 0), g.ny), yn = 3 * miss3(min(o.j + 1, g.ny - 1), g.ny);
+    float rc[4], ra[4], t[4], w4[4], be[4], cu[4], ab[4], so[4], no[4], az[4];
+    auto scaled = [&](const float (&v)[4], int yz, float (&z)[4]) {
+        winv4(w, o, yz, w4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) z[e] = v[e] * w4[e];
+    };
+    ld4(r + c, rc);
+    scaled(rc, yc + miss3(k0, g.nz), cu);
+    ld4(r + (k0 > 0 ? c - sz : c), t);
+    scaled(t, yc + miss3(max(k0 - 1, 0), g.nz), be);
     for (int k = k0; k < k1; ++k, c += sz) {
-        const float above = k + 1 < g.nz ? zat(c + sz, i, j, k + 1) : 0.f;
-        const float az = apply7<float>(g, i, j, k, g.wx, g.wy, g.wz, cur, [&](int a, int b, int e) {
-            return e < 0 ? below : (e > 0 ? above : zat(c + a + b * sy, i + a, j + b, k));
-        });
-        z_out[c] = cur;
-        r_out[c] = r[c] - az;
-        below = cur;
-        cur = above;
+        const bool up = k + 1 < g.nz;
+        const int kc = miss3(k, g.nz);
+        ld4(r + (up ? c + sz : c), ra);
+        scaled(ra, yc + miss3(min(k + 1, g.nz - 1), g.nz), ab);
+        ld4(r + (o.j > 0 ? c - o.sy : c), t);
+        scaled(t, ys + kc, so);
+        ld4(r + (o.j + 1 < g.ny ? c + o.sy : c), t);
+        scaled(t, yn + kc, no);
+        const float mid = w.winv[yc + kc];
+        const float we = o.first ? cu[0] : __ldg(r + c - 1) * mid, ea = o.last ? cu[3] : __ldg(r + c + 4) * mid;
+        apply7x4(g, o, k > 0 ? g.wz : 0.f, up ? g.wz : 0.f, cu, we, ea, so, no, be, ab, az);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            az[e] = rc[e] - az[e];
+            be[e] = cu[e];
+            cu[e] = ab[e];
+            rc[e] = ra[e];
+        }
+        st4(r_out + c, az);
     }
 }
 
-// Post-smoothing of z_in = z_pre + z_net (the coarse correction joins the
-// pre-smoothed part on the fly): z_out = z_in + omega D^-1 (r - A~ z_in).
-__global__ void __launch_bounds__(kBX * kBY) fcg_postsmooth_m(Geo3 g, const float *__restrict__ r,
-                                                              const float *__restrict__ z_pre,
+// Post-smoothing of z_in = z0 + z_net, z0 = omega D^-1 r:
+// z_out = z_in + omega D^-1 (r - A~ z_in).
+__global__ void __launch_bounds__(kBX * kBY) fcg_postsmooth_m(Geo3 g, March m, const float *__restrict__ r,
                                                               const float *__restrict__ z_net, float *z_out,
                                                               const __grid_constant__ SmoothW w) {
-    const int i = blockIdx.x * kBX + (threadIdx.x & 31), j = blockIdx.y * kBY + (threadIdx.x >> 5);
-    const int k0 = blockIdx.z * kMZ, k1 = min(g.nz, k0 + kMZ);
-    if (i >= g.nx || j >= g.ny) return;
-    const long long sy = g.nx, sz = (long long)g.nx * g.ny;
-    long long c = ((long long)k0 * g.ny + j) * g.nx + i;
-    auto zin = [&](long long m) { return z_pre[m] + z_net[m]; };
-    float below = k0 > 0 ? zin(c - sz) : 0.f, cur = zin(c);
+    const Column o = march_column(g, m);
+    const int k0 = blockIdx.y * m.kz, k1 = min(g.nz, k0 + m.kz);
+    if (!o.in) return;
+    const long long sz = (long long)g.nx * g.ny;
+    long long c = o.c + k0 * sz;
+    const int yc = 3 * miss3(o.j, g.ny), ys = 3 * miss3(max(o.j - 1, 0), g.ny), yn = 3 * miss3(min(o.j + 1, g.ny - 1), g.ny);
+    float rc[4], ra[4], t[4], w4[4], be[4], cu[4], ab[4], so[4], no[4], az[4];
+    // z_in of the cells at `at`, r there into rr; the product is rounded before the sum
+    auto zin = [&](long long at, int yz, float (&rr)[4], float (&z)[4]) {
+        ld4(r + at, rr);
+        ld4(z_net + at, z);
+        winv4(w, o, yz, w4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) z[e] = __fadd_rn(__fmul_rn(rr[e], w4[e]), z[e]);
+    };
+    zin(k0 > 0 ? c - sz : c, yc + miss3(max(k0 - 1, 0), g.nz), t, be);
+    zin(c, yc + miss3(k0, g.nz), rc, cu);
     for (int k = k0; k < k1; ++k, c += sz) {
-        const float above = k + 1 < g.nz ? zin(c + sz) : 0.f;
-        const float az = apply7<float>(g, i, j, k, g.wx, g.wy, g.wz, cur, [&](int a, int b, int e) {
-            return e < 0 ? below : (e > 0 ? above : zin(c + a + b * sy));
-        });
-        const float res = r[c] - az;
-        z_out[c] = cur + res * winv_at(w, g, i, j, k);
-        below = cur;
-        cur = above;
+        const bool up = k + 1 < g.nz;
+        const int kc = miss3(k, g.nz);
+        zin(up ? c + sz : c, yc + miss3(min(k + 1, g.nz - 1), g.nz), ra, ab);
+        zin(o.j > 0 ? c - o.sy : c, ys + kc, t, so);
+        zin(o.j + 1 < g.ny ? c + o.sy : c, yn + kc, t, no);
+        const float mid = w.winv[yc + kc];
+        const float we = o.first ? cu[0] : __fadd_rn(__fmul_rn(__ldg(r + c - 1), mid), __ldg(z_net + c - 1));
+        const float ea = o.last ? cu[3] : __fadd_rn(__fmul_rn(__ldg(r + c + 4), mid), __ldg(z_net + c + 4));
+        apply7x4(g, o, k > 0 ? g.wz : 0.f, up ? g.wz : 0.f, cu, we, ea, so, no, be, ab, az);
+        winv4(w, o, yc + kc, w4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            az[e] = cu[e] + (rc[e] - az[e]) * w4[e];
+            be[e] = cu[e];
+            cu[e] = ab[e];
+            rc[e] = ra[e];
+        }
+        st4(z_out + c, az);
     }
 }
 
@@ -391,7 +494,7 @@ int pw_grid(long long n4) { return (int)std::max<long long>(1, std::min<long lon
 struct FcgWork {
     int nx = 0, ny = 0, nz = 0;
     float *r = nullptr, *z = nullptr;
-    float *t1 = nullptr, *t2 = nullptr;  // smoothed residual and coarse correction
+    float *t1 = nullptr;  // smoothed residual
     float *dd[kMaxM] = {}, *qq[kMaxM] = {};  // stored directions and their A~ images
     int ndirs = 0;
     cudaError_t ensure_dirs(int m) {
@@ -417,7 +520,6 @@ struct FcgWork {
         cudaError_t e = cudaMalloc(&r, 4 * n);
         if (e == cudaSuccess) e = cudaMalloc(&z, 4 * n);
         if (e == cudaSuccess) e = cudaMalloc(&t1, 4 * n);
-        if (e == cudaSuccess) e = cudaMalloc(&t2, 4 * n);
         if (e == cudaSuccess) e = cudaMalloc(&partials, sizeof(double) * std::max<long long>(2 * np, kDotStride * kMaxPwBlocks));
         if (e == cudaSuccess) e = cudaMalloc(&sc, sizeof(FcgScalars));
         if (e == cudaSuccess) e = cudaMallocHost(&h_sc, sizeof(FcgScalars));
@@ -430,7 +532,7 @@ struct FcgWork {
         return e;
     }
     void release() {
-        cudaFree(r); cudaFree(z); cudaFree(t1); cudaFree(t2); cudaFree(partials);
+        cudaFree(r); cudaFree(z); cudaFree(t1); cudaFree(partials);
         cudaFree(sc);
         for (int j = 0; j < ndirs; ++j) {
             cudaFree(dd[j]);
@@ -446,7 +548,7 @@ struct FcgWork {
         }
         if (esc) cudaEventDestroy(esc);
         esc = nullptr;
-        r = z = t1 = t2 = nullptr;
+        r = z = t1 = nullptr;
         partials = nullptr;
         sc = h_sc = nullptr;
         nx = ny = nz = 0;
@@ -494,8 +596,13 @@ int32_t fcg_solve(FlursysFcgNet *net, int nx, int ny, int nz, double dx, double 
     const long long n = (long long)nx * ny * nz, n4 = n / 4;
     const dim3 sgrid((nx + kBX - 1) / kBX, (ny + kBY - 1) / kBY, nz), sblock(kBX * kBY);
     const int nsb = (int)(sgrid.x * sgrid.y * sgrid.z), npw = pw_grid(n4);
-    const dim3 mgrid(sgrid.x, sgrid.y, (nz + kMZ - 1) / kMZ);  // z-marching passes
-    const int nmb = (int)(mgrid.x * mgrid.y * mgrid.z);
+    // z-marching passes: up to 16 planes per block, fewer where that would
+    // leave SMs with less than four blocks
+    March march{nx / 4, 16};
+    const int cols = (march.nvec * ny + kBX * kBY - 1) / (kBX * kBY);
+    while (march.kz > 4 && cols * ((nz + march.kz - 1) / march.kz) < 4 * 148) march.kz /= 2;
+    const dim3 mgrid(cols, (nz + march.kz - 1) / march.kz);
+    const int nmb = (int)(mgrid.x * mgrid.y);
     double net_ms = 0.0;
     auto sync_scalars = [&]() -> cudaError_t {
         cudaError_t m = cudaMemcpyAsync(f.h_sc, f.sc, sizeof(FcgScalars), cudaMemcpyDeviceToHost, st);
@@ -541,12 +648,12 @@ int32_t fcg_solve(FlursysFcgNet *net, int nx, int ny, int nz, double dx, double 
             cudaEventRecord(f.e1[pair], st);
             return m;
         }
-        fcg_presmooth_m<<<mgrid, sblock, 0, st>>>(g, f.r, f.t2, f.t1, sw);  // t2 = z0, t1 = r - A z0
+        fcg_presmooth_m<<<mgrid, sblock, 0, st>>>(g, march, f.r, f.t1, sw);  // t1 = r - A z0
         cudaEventRecord(f.e0[pair], st);
         m = net_apply(net->w, net->ws, nx, ny, nz, h2, f.t1, f.z, st);   // z = N(r1)
         cudaEventRecord(f.e1[pair], st);
         if (m != cudaSuccess) return m;
-        fcg_postsmooth_m<<<mgrid, sblock, 0, st>>>(g, f.r, f.t2, f.z, f.t1, sw);  // t1 = post-smoothed z0 + N(r1)
+        fcg_postsmooth_m<<<mgrid, sblock, 0, st>>>(g, march, f.r, f.z, f.t1, sw);  // t1 = post-smoothed z0 + N(r1)
         std::swap(f.z, f.t1);                                                      // z = the preconditioned residual
         return cudaGetLastError();
     };
@@ -609,7 +716,7 @@ int32_t fcg_solve(FlursysFcgNet *net, int nx, int ny, int nz, double dx, double 
             fcg_dots<<<npw, kPw, 0, st>>>(f.z, ds, n4, f.partials);
             fcg_finalize_dots<<<1, 1024, 0, st>>>(f.partials, npw, ds, f.sc, inv_n);
             fcg_direction<<<npw, kPw, 0, st>>>(f.z, dcur, ds, f.sc, n4);
-            fcg_spmv_m<<<mgrid, sblock, 0, st>>>(g, dcur, f.r, qcur, f.partials);
+            fcg_spmv_m<<<mgrid, sblock, 0, st>>>(g, march, dcur, f.r, qcur, f.partials);
             fcg_finalize<<<1, 1024, 0, st>>>(f.partials, nmb, kFinSpmv, f.sc, slot);
             fcg_update<<<npw, kPw, 0, st>>>(x, f.r, dcur, qcur, f.sc, n4, f.partials);
             fcg_finalize<<<1, 1024, 0, st>>>(f.partials, npw, kFinRR, f.sc, 0);
