@@ -124,14 +124,15 @@ def pcg_bytes_per_launch(n_cells: int, iterations: int, precision: str, replace_
     return float(n_cells) * (24 + 80 * iterations + 16)
 
 
-def launches_per_step(iterations: int, precision: str, resident: bool, replace_every: int = 50,
+def launches_per_step(iterations: int, precision: str, one_launch: bool, replace_every: int = 50,
                       unroll: int = 8) -> int:
     """Kernels of one 3D step: predictor (3), rhs, correction, diagnostics (2),
-    and the pressure solve: one cooperative launch when it runs chip-resident;
+    and the pressure solve: one cooperative launch when it runs chip-resident or
+    streams its vectors in one pass;
     otherwise the solve graph's init, operand + update for each iteration of
     every loop body entered (`unroll` iterations per body), fold + replace per
     FP64 replacement, pending fold and final check."""
-    if resident:
+    if one_launch:
         return 7 + 1
     bodies = -(-max(iterations, 1) // unroll)
     nrep = iterations // replace_every + 1 if precision == "mixed" else 0
@@ -399,6 +400,7 @@ def run_ours(args):
     h = _Handle(c)
     h.set_stream(stream.cuda_stream)
     resident = h.solve_kind() == _abi.SOLVE_RESIDENT
+    one_launch = resident or h.solve_kind() == _abi.SOLVE_PERSISTENT
     n_cells = n ** 3
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device=dev)  # > 126 MB L2
 
@@ -461,8 +463,9 @@ def run_ours(args):
             "true_relative_residual_max": max(true_rel),
             "e2e": {"value": e2e_value, "unit": "cell-steps/s", "h2d_bytes_per_step": hbytes,
                     "d2h_bytes_per_step": hbytes + report_bytes},
-            "gpu_launches": sum(launches_per_step(i, precision, resident) for i in its),
-            "pressure_solve": "chip-resident cooperative PCG" if resident else "graph-driven PCG",
+            "gpu_launches": sum(launches_per_step(i, precision, one_launch) for i in its),
+            "pressure_solve": "chip-resident cooperative PCG" if resident else "streaming cooperative PCG" if one_launch
+            else "graph-driven PCG",
             "clocks": clocks,
         }
         line["roofline"] = roofline(n_cells, its, solve_ms, precision, resident)
@@ -726,7 +729,7 @@ def roofline(n_cells, its, solve_ms, precision, resident=False):
            "frac": achieved / peak, "peak_source": peak_src,
            "algorithmic_bytes_per_launch": bytes_total / len(its), "traffic": traffic}
     if resident:
-        out["kernel"] = "pcg3d_res1_kernel (one cooperative launch per solve)"
+        out["kernel"] = "pcg3d_rows_grid (one cooperative launch per solve)"
         out["basis"] = ("HBM-equivalent: compulsory bytes of the streamed MIXED PCG (40 B per cell-iteration) "
                         "over the solve time; the resident kernel's own DRAM traffic is `traffic`")
     else:
