@@ -328,10 +328,17 @@ struct ClusterGroup {
         cluster_barrier();
     }
     __device__ __forceinline__ void finish() { cluster_barrier(); }
+    // Face value for address `a` (of this block; the reader's lies alike) of
+    // block `to`, part of the coming exchange. A buffer is free for it once its
+    // reader has taken part in a round since it last read the buffer.
+    template <typename V>
+    __device__ __forceinline__ void send_to(int to, uint32_t a, V v) const {
+        st_async(cluster_addr(a, to), v, cluster_addr(smem_addr(&sm->fbar[fround & 1u]), to));
+    }
+    // The same for slot h of the buffer of the exchange's parity.
     template <typename V>
     __device__ __forceinline__ void send(int to, int h, V v) const {
-        const uint32_t a = faces + ((fround & 1u) * (uint32_t)face_slots + (uint32_t)h) * (uint32_t)sizeof(V);
-        st_async(cluster_addr(a, to), v, cluster_addr(smem_addr(&sm->fbar[fround & 1u]), to));
+        send_to(to, faces + ((fround & 1u) * (uint32_t)face_slots + (uint32_t)h) * (uint32_t)sizeof(V), v);
     }
     template <typename V>
     __device__ __forceinline__ V face(const V *base, int h) const {

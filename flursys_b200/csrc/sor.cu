@@ -19,6 +19,9 @@
 // not counted. A sweep so takes one round of the
 // group and one exchange with the neighbours. What bounds it is latency: 32^3
 // cells took 19.6 us per sweep with three grid barriers.
+// The even faces that arrive during a sweep's residual pass go to a buffer of
+// their own: a neighbour sends them as soon as it has the odd faces of the sweep
+// before, while this block may still be reading the even ones it then received.
 // sor3d_kernel streams p through L2, with three bounded grid barriers per
 // sweep, for grids whose slabs do not fit.
 #include <cuda_runtime.h>
@@ -133,9 +136,10 @@ constexpr int kResT = 512;
 
 // Cells of one colour in a row, and doubles per plane of one colour.
 __host__ __device__ __forceinline__ int half_row(int nx) { return (nx + 1) / 2; }
-__host__ __device__ __forceinline__ size_t sor_smem(int nx, int ny, int planes) {
+__host__ __device__ __forceinline__ size_t sor_smem(int nx, int ny, int planes, bool cluster) {
     const size_t hp = (size_t)half_row(nx) * ny;
-    return 8 * hp * (5 * (size_t)planes + 4);  // p (the even cells twice) and rhs; two halo planes by colour
+    // p (the even cells twice) and rhs; two halo planes by colour, in a cluster the even ones twice
+    return 8 * hp * (5 * (size_t)planes + (cluster ? 6 : 4));
 }
 
 // a / diag with inv = 1 / diag at hand: the quotient's remainder corrects it
@@ -151,7 +155,7 @@ __device__ __forceinline__ bool sor3d_solve(const SorArgs &a, Group &grp, char *
     const int planes = (nz + grp.nb - 1) / grp.nb, k0 = min(grp.rank * planes, nz), np = min(planes, nz - k0);
     const bool has_lo = np > 0 && k0 > 0, has_hi = np > 0 && k0 + np < nz;
     const double diag = 2.0 * (a.ix2 + a.iy2 + a.iz2), inv = 1.0 / diag;
-    double *P[2], *R[2], *H[2];  // by colour; H: the planes below and above
+    double *P[2], *R[2], *H[2];  // by colour; H: the planes below and above, as read
     P[0] = reinterpret_cast<double *>(dyn);
     double *next_even = P[0] + (size_t)planes * hp;
     P[1] = next_even + (size_t)planes * hp;
@@ -159,11 +163,7 @@ __device__ __forceinline__ bool sor3d_solve(const SorArgs &a, Group &grp, char *
     R[1] = R[0] + (size_t)planes * hp;
     H[0] = R[1] + (size_t)planes * hp;
     H[1] = H[0] + 2 * (size_t)hp;
-    if constexpr (CLUSTER) {
-        // exchange k is colour k & 1's, as are the receive buffers
-        grp.face_slots = 2 * hp;
-        grp.faces = smem_addr(H[0]);
-    }
+    double *next_even_halo = CLUSTER ? H[1] + 2 * (size_t)hp : H[0];  // CLUSTER: where the coming even faces arrive
     // cells of colour c in plane k (a row of parity s = (c + j + k) & 1 holds i = 2 m + s)
     auto count = [&](int c, int k) {
         const int odd_rows = (c + k) & 1 ? (ny + 1) / 2 : ny / 2;  // rows with s = 1
@@ -222,8 +222,14 @@ __device__ __forceinline__ bool sor3d_solve(const SorArgs &a, Group &grp, char *
     };
     auto send = [&](int c, int kk, int j, int m, double v) {
         const int q = j * h + m;
-        if (kk == 0 && has_lo) grp.send(grp.rank - 1, hp + q, v);
-        if (kk == np - 1 && has_hi) grp.send(grp.rank + 1, q, v);
+        if constexpr (CLUSTER) {
+            const uint32_t to = smem_addr(c ? H[1] : next_even_halo);
+            if (kk == 0 && has_lo) grp.send_to(grp.rank - 1, to + 8u * (uint32_t)(hp + q), v);
+            if (kk == np - 1 && has_hi) grp.send_to(grp.rank + 1, to + 8u * (uint32_t)q, v);
+        } else {
+            if (kk == 0 && has_lo) grp.send(grp.rank - 1, hp + q, v);
+            if (kk == np - 1 && has_hi) grp.send(grp.rank + 1, q, v);
+        }
     };
     // the halo planes of colour c from the exchange that has ended (grid form;
     // in the cluster form they are there)
@@ -276,6 +282,9 @@ __device__ __forceinline__ bool sor3d_solve(const SorArgs &a, Group &grp, char *
         double *t = P[0];
         P[0] = next_even;
         next_even = t;
+        t = H[0];
+        H[0] = next_even_halo;
+        next_even_halo = t;
         take_halo(0);
         if (!CLUSTER) __syncthreads();
         // ---- odd cells ----
@@ -339,9 +348,9 @@ constexpr size_t kSorSmemMax = 222 * 1024;
 
 // Blocks of a slab decomposition into at most `most` blocks; 0 where a slab
 // does not fit a block.
-int sor_blocks(int nx, int ny, int nz, int most) {
+int sor_blocks(int nx, int ny, int nz, int most, bool cluster) {
     const int planes = (nz + most - 1) / most;
-    if (sor_smem(nx, ny, planes) > kSorSmemMax) return 0;
+    if (sor_smem(nx, ny, planes, cluster) > kSorSmemMax) return 0;
     return (nz + planes - 1) / planes;
 }
 
@@ -355,9 +364,9 @@ cudaError_t sor3d_plan(Sor3dPlan &plan, int nx, int ny, int nz, int device) {
     int sms = 0;
     cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
-    const int nc = may_cluster ? sor_blocks(nx, ny, nz, 16) : 0;
+    const int nc = may_cluster ? sor_blocks(nx, ny, nz, 16, true) : 0;
     if (nc > 0) {
-        plan.smem = sor_smem(nx, ny, (nz + 15) / 16);
+        plan.smem = sor_smem(nx, ny, (nz + 15) / 16, true);
         if (cudaFuncSetAttribute(sor3d_res_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) == cudaSuccess &&
             cudaFuncSetAttribute(sor3d_res_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cudaLaunchAttribute attr[1];
@@ -379,9 +388,9 @@ cudaError_t sor3d_plan(Sor3dPlan &plan, int nx, int ny, int nz, int device) {
         }
         cudaGetLastError();
     }
-    const int most = std::min(sms, 160), ng = sor_blocks(nx, ny, nz, most);
+    const int most = std::min(sms, 160), ng = sor_blocks(nx, ny, nz, most, false);
     if (ng == 0) return cudaSuccess;
-    plan.smem = sor_smem(nx, ny, (nz + most - 1) / most);
+    plan.smem = sor_smem(nx, ny, (nz + most - 1) / most, false);
     int per_sm = 0;
     if (cudaFuncSetAttribute(sor3d_res_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sor3d_res_grid, kResT, plan.smem) != cudaSuccess || per_sm < 1) {
