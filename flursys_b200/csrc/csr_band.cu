@@ -291,7 +291,9 @@ BandPlan csr_band_plan(long long n, long long band, long long width, int device)
                : width == 7 ? (const void *)cg_band_kernel<7>
                             : (const void *)cg_band_kernel<0>;
     int per_sm = 0;
-    if (cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+    // the limit is the function's, which solves on several threads share:
+    // always the same ceiling, never lowered
+    if (cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBandSmemMax) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, kBandThreads, p.smem) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         return BandPlan{};
@@ -309,11 +311,7 @@ cudaError_t csr_band_launch(const BandPlan &plan, const BandArgs &args, cudaStre
     a.band = plan.band;
     a.width = plan.width;
     void *params[] = {&a};
-    // the limit is the function's; another plan may have set a smaller one
-    cudaError_t e = cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
-    return e == cudaSuccess
-               ? cudaLaunchCooperativeKernel(plan.kernel, dim3(plan.blocks), dim3(kBandThreads), params, plan.smem, stream)
-               : e;
+    return cudaLaunchCooperativeKernel(plan.kernel, dim3(plan.blocks), dim3(kBandThreads), params, plan.smem, stream);
 }
 
 }  // namespace flursys

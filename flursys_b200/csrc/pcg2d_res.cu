@@ -814,8 +814,10 @@ size_t smem_of(int precision, bool xreg, int rows, int nx, bool plain) {
                                                 : res2d_smem<double, CLUSTER>(rows, nx, xreg, plain);
 }
 
-cudaError_t prepare_fn(const void *fn, size_t smem, bool cluster) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// The limit belongs to the function, whose handles may plan and launch on
+// several threads: it is set to the same ceiling each time and never lowered.
+cudaError_t prepare_fn(const void *fn, bool cluster) {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
     if (e == cudaSuccess && cluster) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
@@ -875,7 +877,7 @@ cudaError_t pcg2d_res_plan(Pcg2dResPlan &plan, int nx, int ny, bool plain, int p
             cudaLaunchAttribute attr[1];
             const cudaLaunchConfig_t cfg = cluster_config(nb, nb, variant_threads(plan.variant), plan.smem, nullptr, attr);
             int active = 0;
-            if (prepare_fn(fn, plan.smem, true) == cudaSuccess &&
+            if (prepare_fn(fn, true) == cudaSuccess &&
                 cudaOccupancyMaxActiveClusters(&active, fn, &cfg) == cudaSuccess && active >= 1) {
                 plan.enabled = true;
                 return cudaSuccess;
@@ -893,7 +895,7 @@ cudaError_t pcg2d_res_plan(Pcg2dResPlan &plan, int nx, int ny, bool plain, int p
     const size_t bytes = sizeof(RedRecord) * 2 * plan.nblocks * (kRedSlots + 2 * (size_t)std::max(res2d_pitch<float>(nx), res2d_pitch<double>(nx)));
     const void *fn = res_fn<false>(precision, plan.variant);
     int per_sm = 0;
-    if (prepare_fn(fn, plan.smem, false) != cudaSuccess ||
+    if (prepare_fn(fn, false) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, variant_threads(plan.variant), plan.smem) != cudaSuccess ||
         per_sm < 1) {
         cudaGetLastError();
@@ -922,17 +924,13 @@ cudaError_t pcg2d_res_launch(Pcg2dResPlan &plan, const Pcg2dInstance *inst_dev, 
         cudaLaunchAttribute attr[1];
         const cudaLaunchConfig_t cfg = cluster_config(plan.nblocks, plan.nblocks, threads, plan.smem, stream, attr);
         void *params[] = {&inst_dev};
-        e = prepare_fn(fn, plan.smem, true);
-        return e == cudaSuccess ? cudaLaunchKernelExC(&cfg, fn, params) : e;
+        return cudaLaunchKernelExC(&cfg, fn, params);
     }
     const void *fn = res_fn<false>(plan.precision, plan.variant);
-    e = prepare_fn(fn, plan.smem, false);
     RedRecord *records = plan.records, *faces = plan.records + 2 * (size_t)plan.nblocks * kRedSlots;
     unsigned epoch = ++plan.epoch;
     void *params[] = {&inst_dev, &records, &faces, &epoch};
-    if (e == cudaSuccess)
-        e = cudaLaunchCooperativeKernel(fn, dim3(plan.nblocks), dim3(threads), params, plan.smem, stream);
-    return e;
+    return cudaLaunchCooperativeKernel(fn, dim3(plan.nblocks), dim3(threads), params, plan.smem, stream);
 }
 
 static const void *queue_fn(int precision) {
@@ -956,7 +954,7 @@ cudaError_t pcg2d_queue_plan(Pcg2dQueuePlan &plan, int precision, size_t smem, i
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = cluster_config(kMaxCluster, kMaxCluster, 512, smem, nullptr, attr);
     int active = 0;
-    if (prepare_fn(fn, smem, true) != cudaSuccess ||
+    if (prepare_fn(fn, true) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess || active < 1) {
         cudaGetLastError();
         return cudaSuccess;
@@ -974,8 +972,7 @@ cudaError_t pcg2d_queue_launch(const Pcg2dQueuePlan &plan, const Pcg2dInstance *
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = cluster_config(clusters * plan.nblocks, plan.nblocks, 512, plan.smem, stream, attr);
     void *params[] = {&insts, &order, &count, &next};
-    cudaError_t e = prepare_fn(fn, plan.smem, true);
-    return e == cudaSuccess ? cudaLaunchKernelExC(&cfg, fn, params) : e;
+    return cudaLaunchKernelExC(&cfg, fn, params);
 }
 
 }  // namespace flursys

@@ -871,7 +871,9 @@ bool pcg3d_res_plan(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device) {
     plan.kernel = !plan.single ? (const void *)pcg3d_res2_kernel
                   : plan.col32 ? (const void *)pcg3d_res1_kernel<kResBlock, true>
                                : (const void *)pcg3d_res1_kernel<kResBlock, false>;
-    if (cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) != cudaSuccess)
+    // the limit is the function's, which handles on several threads share:
+    // always that of the deepest tile, never lowered
+    if (cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_smem_bytes(kResMaxTz)) != cudaSuccess)
         return false;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plan.kernel, plan.block, plan.smem) != cudaSuccess ||
         per_sm < 1 || plan.grid > per_sm * sms)

@@ -770,7 +770,9 @@ bool pcg3d_rows_plan(Pcg3dRowsPlan &plan, const Pcg3dArgs &args, int precision, 
     for (;;) {
         if (!(mixed ? choose_rows<float>(plan, sms, may_cluster, true) : choose_rows<double>(plan, sms, may_cluster, true)))
             return false;
-        bool fits = cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) == cudaSuccess;
+        // the limit is the function's, which handles on several threads share:
+        // always the same ceiling, never lowered
+        bool fits = cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmemMax) == cudaSuccess;
         if (fits && plan.cluster) {
             fits = cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
             cudaLaunchAttribute attr[1];
@@ -834,8 +836,6 @@ cudaError_t pcg3d_rows_launch(Pcg3dRowsPlan &plan, CgSeqState *state, cudaStream
         attr[0].id = cudaLaunchAttributeCooperative;
         attr[0].val.cooperative = 1;
     }
-    // the limit is the function's; another handle may have set a smaller one
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
     return e == cudaSuccess ? cudaLaunchKernelExC(&cfg, plan.kernel, params) : e;
 }
 

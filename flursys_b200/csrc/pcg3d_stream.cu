@@ -714,7 +714,9 @@ bool pcg3d_stream_plan(Pcg3dStreamPlan &plan, const Pcg3dArgs &args, int precisi
     if (!(mixed ? choose_stream<float>(plan, most) : choose_stream<double>(plan, most))) return false;
     const size_t bytes = (mixed ? 4 * (size_t)row_pitch<float>(a.nx) : 8 * (size_t)row_pitch<double>(a.nx)) * a.ny * a.nz;
     const size_t rec = sizeof(RedRecord) * 2 * plan.blocks * kRedSlots;
-    if (cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) != cudaSuccess ||
+    // (the limit is the function's, which handles on several threads share:
+    // always the same ceiling, never lowered)
+    if (cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmemMax) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plan.kernel, kT, plan.smem) != cudaSuccess || per_sm < 1 ||
         cudaMalloc(&plan.records, rec) != cudaSuccess || cudaMemset(plan.records, 0, rec) != cudaSuccess ||
         cudaStreamSynchronize(nullptr) != cudaSuccess ||  // solves run on streams that do not wait for this one
@@ -740,8 +742,6 @@ cudaError_t pcg3d_stream_launch(Pcg3dStreamPlan &plan, CgSeqState *state, cudaSt
     a.fault = take_injected_barrier_fault();
     cudaError_t e = cudaMemsetAsync(state, 0, sizeof(CgSeqState), stream);
     void *params[] = {&a};
-    // the limit is the function's; another handle may have set a smaller one
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
     return e == cudaSuccess
                ? cudaLaunchCooperativeKernel(plan.kernel, dim3(plan.blocks), dim3(kT), params, plan.smem, stream)
                : e;

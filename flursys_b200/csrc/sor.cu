@@ -367,7 +367,9 @@ cudaError_t sor3d_plan(Sor3dPlan &plan, int nx, int ny, int nz, int device) {
     const int nc = may_cluster ? sor_blocks(nx, ny, nz, 16, true) : 0;
     if (nc > 0) {
         plan.smem = sor_smem(nx, ny, (nz + 15) / 16, true);
-        if (cudaFuncSetAttribute(sor3d_res_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) == cudaSuccess &&
+        // the limit is the function's, which handles on several threads share:
+        // always the same ceiling, never lowered
+        if (cudaFuncSetAttribute(sor3d_res_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSorSmemMax) == cudaSuccess &&
             cudaFuncSetAttribute(sor3d_res_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -392,7 +394,7 @@ cudaError_t sor3d_plan(Sor3dPlan &plan, int nx, int ny, int nz, int device) {
     if (ng == 0) return cudaSuccess;
     plan.smem = sor_smem(nx, ny, (nz + most - 1) / most, false);
     int per_sm = 0;
-    if (cudaFuncSetAttribute(sor3d_res_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) != cudaSuccess ||
+    if (cudaFuncSetAttribute(sor3d_res_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSorSmemMax) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sor3d_res_grid, kResT, plan.smem) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         return cudaSuccess;
@@ -437,8 +439,6 @@ int32_t run_sor3d(Sor3dPlan &plan, PcgWorkspace &ws, int nx, int ny, int nz, dou
             attr[0].id = cudaLaunchAttributeCooperative;
             attr[0].val.cooperative = 1;
         }
-        // the limit is the function's; another handle may have set a smaller one
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
         if (e == cudaSuccess) e = cudaLaunchKernelExC(&cfg, fn, params);
         if (e != cudaSuccess) return set_cuda_error(err, e, "sor3d launch");
         return FLURSYS_OK;
