@@ -448,6 +448,48 @@ float time_ms(FlursysBatchHandle *h, int reps, F fn, cudaError_t *e) {
     return ms / reps;
 }
 
+// Where a batch has instances that the queue cannot take (SOR, too large a
+// grid), the cooperative launch runs after the queue, and an instance that
+// would share it costs little there: the index in `order` (largest first) from
+// which on instances are queued so that both launches together take least time.
+// A queued iteration takes about 2.9 us + 42 ps per cell on its cluster; the
+// cooperative launch takes 15.8 (F64: 12.2) us for each iteration of its
+// longest instance and 14.2 (19) ps for each cell and iteration of any. Per
+// step in MIXED, all that fit queued and as chosen here: 512^2 + 520^2 63 and
+// 46 ms, 512^2 + 600^2 76 and 53, eight 64^2 + 600^2 52 and 49, three 448^2 +
+// three 600^2 89 and 81. (A batch that fits the queue as a whole is 1.5 to 3.9
+// times faster there at any count.)
+int queue_from(const FlursysBatchHandle *h, const std::vector<int> &order) {
+    const bool mixed = h->precision == FLURSYS_PRECISION_MIXED;
+    const double base = mixed ? 15.8 : 12.2, per_cell = mixed ? 14.2e-6 : 19.0e-6;
+    // iterations grow with the longer side; SOR needs several times as many
+    auto its = [&](int i) { return double(std::max(h->nx[i], h->ny[i])) * (h->h_pin[i].solver == FLURSYS_PRESSURE_SOR ? 8.0 : 1.0); };
+    auto cells = [&](int i) { return double(h->h_ctl[i].cells); };
+    double longest = 0.0, work = 0.0;  // of the cooperative launch
+    for (int i = 0; i < h->n; ++i)
+        if (std::find(order.begin(), order.end(), i) == order.end()) {
+            longest = std::max(longest, its(i));
+            work += cells(i) * its(i);
+        }
+    int best_first = 0;
+    double best = 0.0;
+    for (int first = 0; first <= (int)order.size(); ++first) {
+        std::vector<double> busy(h->queue.clusters, 0.0);
+        for (int k = first; k < (int)order.size(); ++k)
+            *std::min_element(busy.begin(), busy.end()) += its(order[k]) * (2.9 + 42.0e-6 * cells(order[k]));
+        const double t = *std::max_element(busy.begin(), busy.end()) + base * longest + per_cell * work;
+        if (first == 0 || t < best) {
+            best = t;
+            best_first = first;
+        }
+        if (first < (int)order.size()) {
+            longest = std::max(longest, its(order[first]));
+            work += cells(order[first]) * its(order[first]);
+        }
+    }
+    return best_first;
+}
+
 cudaError_t autotune(FlursysBatchHandle *h) {
     cudaError_t e = cudaSuccess;
     // tile kernels: every op is idempotent on the initial state
@@ -711,15 +753,27 @@ extern "C" int32_t flursys_cuda_batch_create(const FlursysCudaConfig *configs, i
     // the other clusters idle); the rest share the cooperative launch.
     std::vector<int> order;
     if (e == cudaSuccess) {
-        size_t smem = 0, need = 0;
+        size_t need = 0;
+        std::vector<size_t> smem(count, 0);
+        auto plan = [&]() {
+            size_t most = 0;
+            for (int i : order) most = std::max(most, smem[i]);
+            h->queue = Pcg2dQueuePlan{};
+            if (!order.empty()) e = pcg2d_queue_plan(h->queue, h->precision, most, h->device);
+            if (!h->queue.clusters) order.clear();
+        };
         for (int i = 0; i < count; ++i)
             if (h->h_pin[i].solver == FLURSYS_PRESSURE_PCG && pcg2d_queue_fits(h->nx[i], h->ny[i], h->h_pin[i].count_fluid == h->h_ctl[i].cells, h->precision, &need)) {
-                smem = std::max(smem, need);
+                smem[i] = need;
                 order.push_back(i);
             }
-        if (!order.empty()) e = pcg2d_queue_plan(h->queue, h->precision, smem, h->device);
-        if (!h->queue.clusters) order.clear();
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->h_ctl[a].cells > h->h_ctl[b].cells; });
+        plan();
+        if (e == cudaSuccess && !order.empty() && (int)order.size() < count) {
+            const int first = queue_from(h, order);
+            order.erase(order.begin(), order.begin() + first);
+            if (first > 0) plan();
+        }
         for (int i : order) h->h_pin[i].resident = 1;
         h->queued = (int)order.size();
         if (e == cudaSuccess && h->queued)
