@@ -44,14 +44,28 @@ constexpr int kRoundCols = 8;
 constexpr int kParts = 2 * kRoundCols;
 constexpr int kU = 4;  // cells per thread per step of the plain-operator passes
 
-// Barriers between the passes of one instance: the bounded software grid
-// barrier over the instance's blocks.
+// Barriers between the passes of one instance. GridSync: the bounded
+// software grid barrier over the instance's blocks. ClusterSync (SOR): the
+// instance runs as one thread-block cluster and the passes are separated by
+// the hardware cluster barrier (release / acquire at cluster scope, so
+// everything written before it is visible after it in every block of the
+// cluster). Either way the blocks' partial sums meet in global memory, read
+// through L2.
 struct GridSync {
     GridBarrier *bar;
     unsigned nb;
     double *partials;
     unsigned *report;  // the instance's PcgResultDev::device_error
     __device__ __forceinline__ bool operator()() const { return grid_sync_report(bar, nb, report); }
+    __device__ __forceinline__ void put(int lb, int col, double v) const { partials[lb * kParts + col] = v; }
+    __device__ __forceinline__ double get(int b, int col) const { return __ldcg(partials + b * kParts + col); }
+};
+struct ClusterSync {
+    double *partials;
+    __device__ __forceinline__ bool operator()() const {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
     __device__ __forceinline__ void put(int lb, int col, double v) const { partials[lb * kParts + col] = v; }
     __device__ __forceinline__ double get(int b, int col) const { return __ldcg(partials + b * kParts + col); }
 };
@@ -625,6 +639,28 @@ __global__ void __launch_bounds__(kBlock, 3) pcg2d_kernel(const Pcg2dInstance *_
     else pcg_instance<V, MIXED>(k, red, sync);
 }
 
+// SOR of one instance as one thread-block cluster (grid = cluster = nblocks).
+__global__ void __launch_bounds__(kBlock, 3) sor2d_cluster_kernel(const Pcg2dInstance *__restrict__ inst) {
+    __shared__ double red[kRoundCols * (kBlock / 32)];
+    Ctx k;
+    make_ctx(k, inst[0], (int)blockIdx.x);
+    sor_instance(k, red, ClusterSync{k.in.partials});
+}
+
+cudaLaunchConfig_t sor2d_cluster_config(int nblocks, cudaStream_t stream, cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nblocks);
+    cfg.blockDim = dim3(kBlock);
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = nblocks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 }  // namespace
 
 cudaError_t pcg2d_max_grid(int precision, int device, int *grid) {
@@ -638,6 +674,27 @@ cudaError_t pcg2d_max_grid(int precision, int device, int *grid) {
     if (e != cudaSuccess) return e;
     *grid = sms * per_sm;
     return cudaSuccess;
+}
+
+int sor2d_max_cluster() {
+    if (cudaFuncSetAttribute(sor2d_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return 8;  // the portable cluster size
+    }
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = sor2d_cluster_config(16, nullptr, attr);
+    int size = 0;
+    if (cudaOccupancyMaxPotentialClusterSize(&size, sor2d_cluster_kernel, &cfg) != cudaSuccess || size < 1) {
+        cudaGetLastError();
+        return 8;
+    }
+    return size;
+}
+
+cudaError_t sor2d_launch_cluster(const Pcg2dInstance *inst_dev, int nblocks, cudaStream_t stream) {
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = sor2d_cluster_config(nblocks, stream, attr);
+    return cudaLaunchKernelEx(&cfg, sor2d_cluster_kernel, inst_dev);
 }
 
 int pcg2d_block_size() { return kBlock; }

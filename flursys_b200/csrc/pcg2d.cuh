@@ -47,4 +47,10 @@ int pcg2d_num_partials();
 // Launches one cooperative grid over all instances (device array `inst`).
 cudaError_t pcg2d_launch(const Pcg2dInstance *inst_dev, int ninst, int total_blocks, int precision,
                          cudaStream_t stream);
+// Largest thread-block cluster of the 2D SOR (16 where the device allows
+// non-portable sizes, else 8).
+int sor2d_max_cluster();
+// Launches one SOR instance (device pointer) as a single cluster of `nblocks`
+// blocks.
+cudaError_t sor2d_launch_cluster(const Pcg2dInstance *inst_dev, int nblocks, cudaStream_t stream);
 }  // namespace flursys
