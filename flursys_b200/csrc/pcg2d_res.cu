@@ -23,11 +23,14 @@
 // x itself is projected once at the end: A annihilates constants, so these
 // shifts are rounding-sized and change no iterate.
 //
-// MIXED: r, q and d are FP32 with alpha, beta rounded to FP32 (the same alpha
-// for x and r); every product of the inner products is formed and summed in
-// FP64, x is FP64, and r is replaced by the FP64 b - A x every replace_every
-// iterations and before convergence is accepted (d then exchanges M r_old for
-// M r_new, and the operator pass is repeated).
+// MIXED: r, q and d are FP32; alpha, beta, the means and 1/diagonal are FP64, r
+// and d are updated in FP64 and rounded as they are stored, and so is every
+// product of the inner products formed and summed. x is FP64, and r is replaced
+// by the FP64 b - A x every replace_every iterations and before convergence is
+// accepted (d then exchanges M r_old for M r_new, and the operator pass is
+// repeated). (With scalars, weights and updates in FP32 an iteration on 509 x
+// 331 took 5.5 us instead of 5.9, and a solve to 1e-12 2761 of them instead of
+// 2563.)
 //
 // What bounds it: on small grids latency (the block reduction, the exchange,
 // the scalars' chain), on large ones instruction issue. A lane takes 16 bytes
@@ -58,8 +61,16 @@ namespace {
 
 __device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double vfma(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double vadd(double a, double b) { return __dadd_rn(a, b); }
+// r - alpha q less its mean, and M r + shift + beta d, as they are stored: the
+// owner of a cell and the halo copies of it form the same bits.
+template <typename V>
+__device__ __forceinline__ V next_r(double alpha, V q, V r, double mean) {
+    return V(__dadd_rn(__fma_rn(-alpha, double(q), double(r)), -mean));
+}
+template <typename V>
+__device__ __forceinline__ V next_d(double beta, V d, V r, double inv, double shift) {
+    return V(__fma_rn(beta, double(d), __fma_rn(double(r), inv, shift)));
+}
 
 enum : unsigned { kE = 1, kW = 2, kN = 4, kS = 8, kFluid = 16 };
 
@@ -75,13 +86,13 @@ __host__ __device__ __forceinline__ int res2d_pitch(int nx) {
 }
 
 // Shared-memory footprint of a block that owns `rows` grid rows: r, q and d
-// with its halo rows, the halo's r, 1/diagonal and (cluster) two sets of
+// with its halo rows, the halo's r, coupling bits and (cluster) two sets of
 // received faces, x unless it is in registers, and the coupling bits unless
 // every cell is fluid.
 template <typename V, bool CLUSTER>
 __host__ __device__ size_t res2d_smem(int rows, int nx, bool xreg, bool plain) {
     const size_t p = res2d_pitch<V>(nx), c = (size_t)rows * p;
-    size_t b = (xreg ? 0 : 8 * c) + sizeof(V) * (3 * c + (CLUSTER ? 10 : 6) * p + 2 * kVec<V>);
+    size_t b = (xreg ? 0 : 8 * c) + sizeof(V) * (3 * c + (CLUSTER ? 8 : 4) * p + 2 * kVec<V>) + 2 * p;
     if (!plain) b += c;
     return (b + 15) & ~size_t(15);
 }
@@ -107,20 +118,15 @@ struct Res2dGroup<T, true> {
     using type = ClusterGroup<T>;
 };
 
-// 1 / diagonal by coupling bits; 0 marks a row that is not fluid. `d` holds the
-// values of `v` widened.
-template <typename V>
+// 1 / diagonal by coupling bits; 0 marks a row that is not fluid.
 struct Res2dTable {
-    V v[32];
-    double d[32];
+    double inv[32];
 };
 
 // What warp 0 hands the block after an iteration's reduction.
 enum : int { kStep = 0, kStop = 1, kRefresh = 2, kFail = 3 };
-template <typename V>
 struct Res2dScalars {
-    double ax, md;             // x += ax (d - md)
-    V alpha, mr, beta, shift;  // r -= alpha q + mr; d = M r + beta d + shift
+    double alpha, md, mr, beta, shift;  // x += alpha (d - md); r -= alpha q + mr; d = M r + beta d + shift
     int cmd;
 };
 
@@ -147,7 +153,7 @@ __device__ __forceinline__ unsigned cell_bits(const Pcg2dInstance &in, bool plai
 // fluid.
 template <typename V, int T, int XN, bool CLUSTER, bool PLAIN>
 __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Res2dGroup<T, CLUSTER>::type &grp,
-                                            char *dyn, Res2dTable<V> &tab, Res2dScalars<V> &sc) {
+                                            char *dyn, Res2dTable &tab, Res2dScalars &sc) {
     constexpr bool MIXED = sizeof(V) == 4;
     constexpr int W = kVec<V>, U = 4 / W;  // cells per vector, vectors per trip
     constexpr int XV = (XN + W - 1) / W;   // vectors of x in registers
@@ -168,9 +174,9 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
     V *qs = rs + cpad;
     V *ds = qs + cpad;
     V *hr = ds + cpad + 2 * (size_t)P + 2 * W;  // halo: [below, above][P]
-    V *hm = hr + 2 * (size_t)P;
-    V *hq = hm + 2 * (size_t)P;  // CLUSTER: face values received, by round parity
-    uint8_t *bs = reinterpret_cast<uint8_t *>(hq + (CLUSTER ? 4 * (size_t)P : 0));
+    V *hq = hr + 2 * (size_t)P;  // CLUSTER: face values received, by round parity
+    uint8_t *hb = reinterpret_cast<uint8_t *>(hq + (CLUSTER ? 4 * (size_t)P : 0));  // the halo's coupling bits
+    uint8_t *bs = hb + 2 * (size_t)P;
     V *const dc0 = ds + P + W;  // d of cell (0, 0)
     if constexpr (CLUSTER) {
         grp.face_slots = 2 * P;
@@ -181,9 +187,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
 
     if (tid < 32) {  // 1 / diagonal by coupling bits; 0 marks a row that is not fluid
         const double dg = double((tid & 1) + ((tid >> 1) & 1)) * in.idx2 + double(((tid >> 2) & 1) + ((tid >> 3) & 1)) * in.idy2;
-        const V m = (tid & kFluid) ? (dg > 0.0 ? V(1.0 / dg) : V(1)) : V(0);
-        tab.v[tid] = m;
-        tab.d[tid] = double(m);
+        tab.inv[tid] = (tid & kFluid) ? (dg > 0.0 ? 1.0 / dg : 1.0) : 0.0;
     }
     for (int k = tid; k < (int)cpad + 2 * P + 2 * W; k += T) ds[k] = V(0);
     for (int k = tid; k < (int)cpad; k += T) rs[k] = qs[k] = V(0);
@@ -297,7 +301,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                 if (k > 1) grp.peek(h, tv, tt);
                 v = V(grp.take(h, tv, tt));
             }
-            if (PLAIN || hm[h] != V(0)) f(h, hd(h), v);
+            if (PLAIN || (hb[h] & kFluid)) f(h, hd(h), v);
         }
     };
 
@@ -307,7 +311,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
         return __ldcg(in.x + g);
     };
 
-    // ---- set-up: bits, x, the halo's 1/diagonal; sums of x and b ----
+    // ---- set-up: bits, x, the halo's bits; sums of x and b ----
     clear();
     if (!PLAIN) {
         for (int row = wid; row < nr; row += NW)
@@ -325,7 +329,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
     for (int t = tid; t < nh; t += T) {
         const int h = hslot(t), g = h < P ? (j0 - 1) * nx + h : (j0 + nr) * nx + h - P;
         hr[h] = V(0);
-        hm[h] = tab.v[cell_bits(in, PLAIN, g)];
+        hb[h] = (uint8_t)cell_bits(in, PLAIN, g);
     }
     if (!grp.all(s, false)) return false;
     const double mb = proj ? s[1] / cnt : 0.0;
@@ -348,7 +352,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
         clear();
         each_cell([&](int row, int i, int o, unsigned b) {
             if (!(b & kFluid)) return;
-            if (fix) dc0[o] = vfma(-rs[o], tab.v[b], dc0[o]);
+            if (fix) dc0[o] = V(fma(-double(rs[o]), tab.inv[b], double(dc0[o])));
             const double rv = true_residual(row, i, b);
             s[0] += rv;
             rs[o] = V(rv);
@@ -356,7 +360,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
         if (fix)
             for (int t = tid; t < nh; t += T) {
                 const int h = hslot(t);
-                hd(h) = vfma(-hr[h], hm[h], hd(h));
+                hd(h) = V(fma(-double(hr[h]), tab.inv[hb[h]], double(hd(h))));
             }
         if (!grp.all(s, false)) return false;
         const double mr = proj ? s[0] / cnt : 0.0;
@@ -365,8 +369,8 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
             if (!(b & kFluid)) return;
             const V rv = V(double(rs[o]) - mr);
             rs[o] = rv;
-            if (fix) put_d(row, i, o, vfma(rv, tab.v[b], dc0[o]));
-            const double rd = double(rv), zd = rd * tab.d[b];
+            const double rd = double(rv), zd = rd * tab.inv[b];
+            if (fix) put_d(row, i, o, V(fma(rd, tab.inv[b], double(dc0[o]))));
             s[1] = fma(rd, zd, s[1]);
             s[4] += rd;
             s[5] += zd;
@@ -379,7 +383,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
         peek_halo();
         each_halo([&](int h, V &d, V v) {
             hr[h] = v;
-            if (fix) d = vfma(v, hm[h], d);
+            if (fix) d = V(fma(double(v), tab.inv[hb[h]], double(d)));
         });
         return true;
     };
@@ -418,13 +422,13 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
             }
             if (__syncthreads_or(tid < 32 && last)) break;
             if (it == 0) {  // d = M r less its mean
-                const V shift = V(proj ? -s[5] / cnt : 0.0);
+                const double shift = proj ? -s[5] / cnt : 0.0;
                 each_cell([&](int row, int i, int o, unsigned b) {
-                    if (b & kFluid) put_d(row, i, o, vfma(rs[o], tab.v[b], shift));
+                    if (b & kFluid) put_d(row, i, o, V(fma(double(rs[o]), tab.inv[b], shift)));
                 });
                 for (int t = tid; t < nh; t += T) {
                     const int h = hslot(t);
-                    if (hm[h] != V(0)) hd(h) = vfma(hr[h], hm[h], shift);
+                    if (hb[h] & kFluid) hd(h) = V(fma(double(hr[h]), tab.inv[hb[h]], shift));
                 }
             } else {
                 replaced = true;
@@ -466,13 +470,13 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                         qc[k] = vfma(wx, (dc[u][k] - e) + (dc[u][k] - wv),
                                      wy * ((dc[u][k] - no[u][k]) + (dc[u][k] - so[u][k])));
                     }
-                    const double mi = tab.d[row_bits(row[u]) | kE | kW];
+                    const double mi = tab.inv[row_bits(row[u]) | kE | kW];
 #pragma unroll
                     for (int k = 0; k < W; ++k) md[k] = mi;
                     if (v[u] == 0 || v[u] == nvec - 1) {
 #pragma unroll
                         for (int k = 0; k < W; ++k) {
-                            if (i + k == 0 || i + k == nx - 1) md[k] = tab.d[row_bits(row[u]) | col_bits(i + k)];
+                            if (i + k == 0 || i + k == nx - 1) md[k] = tab.inv[row_bits(row[u]) | col_bits(i + k)];
                             if (i + k >= nx) qc[k] = dc[u][k] = V(0);  // behind the row
                         }
                     }
@@ -484,7 +488,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                         const V de = (b & kE) ? c - e : V(0), dw = (b & kW) ? c - wv : V(0);
                         const V dn = (b & kN) ? c - no[u][k] : V(0), dso = (b & kS) ? c - so[u][k] : V(0);
                         qc[k] = vfma(wx, de + dw, wy * (dn + dso));
-                        md[k] = tab.d[b];
+                        md[k] = tab.inv[b];
                     }
                 }
                 stv(qs + o, qc);
@@ -546,12 +550,11 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                 rz_old = rz;
             }
             if (tid == 0) {
-                sc.alpha = V(alpha);
-                sc.ax = double(V(alpha));
+                sc.alpha = alpha;
                 sc.md = md;
-                sc.mr = V(mr);
-                sc.beta = V(beta);
-                sc.shift = V(-mz - beta * md);
+                sc.mr = mr;
+                sc.beta = beta;
+                sc.shift = -mz - beta * md;
                 sc.cmd = cmd;
             }
         }
@@ -569,8 +572,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
             continue;
         }
         replaced = false;
-        const V av = sc.alpha, mrv = sc.mr, bv = sc.beta, shift = sc.shift;
-        const double ax = sc.ax, md = sc.md;
+        const double alpha = sc.alpha, mr = sc.mr, beta = sc.beta, shift = sc.shift, md = sc.md;
         if constexpr (XN > 0) {  // a vector of x at a time; values behind a row are never used
             Walk w = first();
             asm volatile("" : "+r"(w.row), "+r"(w.strip));
@@ -581,7 +583,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                     V dc[W];
                     ldv(dc0 + w.row * P + v * W, dc);
 #pragma unroll
-                    for (int k = 0; k < W; ++k) xr[u * W + k] = fma(ax, double(dc[k]) - md, xr[u * W + k]);
+                    for (int k = 0; k < W; ++k) xr[u * W + k] = fma(alpha, double(dc[k]) - md, xr[u * W + k]);
                 }
                 next(w);
             }
@@ -604,21 +606,22 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
             for (int u = 0; u < U; ++u) {
                 if (v[u] < 0) continue;
                 const int i = v[u] * W, o = row[u] * P + i;
-                V dn[W], inv[W];
+                V dn[W];
+                double inv[W];
                 unsigned b[W];
                 const unsigned rb = row_bits(row[u]);
-                const V ii = tab.v[rb | kE | kW];
+                const double ii = tab.inv[rb | kE | kW];
 #pragma unroll
                 for (int k = 0; k < W; ++k) {
                     b[k] = PLAIN ? 31u : (unsigned)bs[o + k];
-                    inv[k] = PLAIN ? ii : tab.v[b[k]];
+                    inv[k] = PLAIN ? ii : tab.inv[b[k]];
                 }
                 const bool edge = v[u] == 0 || v[u] == nvec - 1;
                 if (PLAIN && edge) {
 #pragma unroll
                     for (int k = 0; k < W; ++k) {
                         b[k] = i + k < nx ? 31u : 0u;
-                        if (i + k < nx) inv[k] = tab.v[rb | col_bits(i + k)];
+                        if (i + k < nx) inv[k] = tab.inv[rb | col_bits(i + k)];
                     }
                 }
                 if (XN == 0) {
@@ -626,15 +629,15 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                     for (int k = 0; k < W; k += 2) {  // x of two cells per 16-byte access
                         double2 *xp = reinterpret_cast<double2 *>(xs + o + k);
                         double2 xv = *xp;
-                        xv.x = fma(ax, double(dc[u][k]) - md, xv.x);
-                        xv.y = fma(ax, double(dc[u][k + 1]) - md, xv.y);
+                        xv.x = fma(alpha, double(dc[u][k]) - md, xv.x);
+                        xv.y = fma(alpha, double(dc[u][k + 1]) - md, xv.y);
                         *xp = xv;
                     }
                 }
 #pragma unroll
                 for (int k = 0; k < W; ++k) {
-                    const V rn = vadd(vfma(-av, qv[u][k], rv[u][k]), -mrv);
-                    dn[k] = vfma(bv, dc[u][k], vfma(rn, inv[k], shift));
+                    const V rn = next_r(alpha, qv[u][k], rv[u][k], mr);
+                    dn[k] = next_d(beta, dc[u][k], rn, inv[k], shift);
                     rv[u][k] = (b[k] & kFluid) ? rn : V(0);
                     if (!(b[k] & kFluid)) dn[k] = V(0);
                 }
@@ -657,9 +660,9 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
             }
         }
         each_halo([&](int h, V &d, V qv) {
-            const V hn = vadd(vfma(-av, qv, hr[h]), -mrv);
+            const V hn = next_r(alpha, qv, hr[h], mr);
             hr[h] = hn;
-            d = vfma(bv, d, vfma(hn, hm[h], shift));
+            d = next_d(beta, d, hn, tab.inv[hb[h]], shift);
         });
         ++it;
         ++since;
@@ -701,7 +704,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
 
 template <typename V, int T, int XN, bool CLUSTER>
 __device__ __forceinline__ bool res2d_run(const Pcg2dInstance &in, typename Res2dGroup<T, CLUSTER>::type &grp,
-                                          char *dyn, Res2dTable<V> &tab, Res2dScalars<V> &sc) {
+                                          char *dyn, Res2dTable &tab, Res2dScalars &sc) {
     if (in.count_fluid == (long long)in.nx * in.ny) return res2d_solve<V, T, XN, CLUSTER, true>(in, grp, dyn, tab, sc);
     return res2d_solve<V, T, XN, CLUSTER, false>(in, grp, dyn, tab, sc);
 }
@@ -710,8 +713,8 @@ template <typename V, int T, int XN>
 __global__ void __launch_bounds__(T, 1) pcg2d_res_cluster(const Pcg2dInstance *__restrict__ inst) {
     extern __shared__ __align__(16) char dyn[];
     __shared__ ClusterRedShared<T> red;
-    __shared__ Res2dTable<V> tab;
-    __shared__ Res2dScalars<V> sc;
+    __shared__ Res2dTable tab;
+    __shared__ Res2dScalars sc;
     __shared__ Pcg2dInstance in;
     if (threadIdx.x == 0) in = inst[0];
     __syncthreads();
@@ -727,8 +730,8 @@ __global__ void __launch_bounds__(T, 1) pcg2d_res_grid(const Pcg2dInstance *__re
                                                        RedRecord *faces, unsigned epoch) {
     extern __shared__ __align__(16) char dyn[];
     __shared__ GridRedShared<T> red;
-    __shared__ Res2dTable<V> tab;
-    __shared__ Res2dScalars<V> sc;
+    __shared__ Res2dTable tab;
+    __shared__ Res2dScalars sc;
     __shared__ Pcg2dInstance in;
     if (threadIdx.x == 0) {
         in = inst[0];
@@ -746,8 +749,8 @@ __global__ void __launch_bounds__(T, 1) pcg2d_res_queue(const Pcg2dInstance *__r
                                                         const int *__restrict__ order, int count, unsigned *next) {
     extern __shared__ __align__(16) char dyn[];
     __shared__ ClusterRedShared<T> red;
-    __shared__ Res2dTable<V> tab;
-    __shared__ Res2dScalars<V> sc;
+    __shared__ Res2dTable tab;
+    __shared__ Res2dScalars sc;
     __shared__ Pcg2dInstance in;
     __shared__ int slot, gave_up;
     int nb, rank;
