@@ -212,9 +212,9 @@ __global__ void __launch_bounds__(kBandThreads, 1) cg_band_kernel(const __grid_c
                 }
                 if (!stop) {
                     const bool plain = fabs(den) < big && fabs(rz) < big;
-                    const double alpha = plain ? rz * fast_recip(den) : rz / den;
+                    const double alpha = plain ? quotient(rz, den, fast_recip(den)) : rz / den;
                     double beta = rz + alpha * (alpha * s[3] - 2.0 * s[2]);
-                    beta = plain && fabs(rz) > 1.0e-300 ? beta * fast_recip(rz) : beta / rz;
+                    beta = plain && fabs(rz) > 1.0e-300 ? quotient(beta, rz, fast_recip(rz)) : beta / rz;
                     if (!isfinite(den)) error = FLURSYS_ERR_NON_FINITE;
                     else if (fabs(den) <= 1.0e-30 || !isfinite(alpha)) error = FLURSYS_ERR_BREAKDOWN;
                     if (error) stop = 1;

@@ -125,16 +125,32 @@ __device__ __forceinline__ void spread8(double t, double (&v)[kRedSlots]) {
     for (int k = 0; k < kRedSlots; ++k) v[k] = __shfl_sync(0xffffffffu, t, 4 * k);
 }
 
-// 1 / x by two of Newton's iterations on the hardware's approximate reciprocal
-// (relative error 2^-23, then 2^-46, then rounding), in place of a division's
-// subroutine. For x whose reciprocal is a normal number the error is within a
-// few units in the last place.
+// 1 / x by the Newton-Raphson iteration y + y (1 - x y), which squares the
+// relative error, from the hardware's approximate reciprocal, whose result has
+// 20 bits behind the point: about 2^-20, 2^-40, then rounding. For x and 1 / x
+// that are normal numbers the error is within two units in the last place.
 __device__ __forceinline__ double fast_recip(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
 #pragma unroll
     for (int k = 0; k < 2; ++k) y = fma(y, fma(-x, y, 1.0), y);
     return y;
+}
+// a / b from y, nearly 1 / b: the remainder of the product corrects it
+// (Markstein 1990), which leaves no more than one unit in the last place. With
+// fast_recip() it replaces a division's subroutine in the scalars' chain (three
+// divisions and a square root took about 1000 of an iteration's 5000 cycles on
+// 128^2). Where a / b is infinite or undefined the result is not finite either.
+__device__ __forceinline__ double quotient_step(double q, double a, double b, double y) { return fma(fma(-q, b, a), y, q); }
+__device__ __forceinline__ double quotient(double a, double b, double y) { return quotient_step(a * y, a, b, y); }
+// a / b rounded as the division rounds it, from y = 1 / b so rounded: the
+// second correction starts within one unit in the last place, where Markstein's
+// theorem gives the rounded quotient (remainders below the normal range apart).
+// An a that is not finite, or too large for a / b, gives what a y is.
+__device__ __forceinline__ double rounded_quotient(double a, double b, double y) {
+    const double q = a * y;
+    if (!(fabs(q) <= 1.7976931348623157e308)) return q;
+    return quotient_step(quotient_step(q, a, b, y), a, b, y);
 }
 
 // Hands warp 0's totals and its verdict to the block.

@@ -513,11 +513,11 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
         send_faces(qs);
         const bool ok = grp.lead(s, linf, true, face_bytes, peek_halo);
         if (tid < 32) {  // warp 0: the step's scalars, and the verdict on the current iterate
-            const double den = s[0], iden = fast_recip(den);
+            const double den = s[0];
             const double mz = s[5] * inv_cnt, md = s[6] * inv_cnt, mr = s[4] * inv_cnt;
             const double rz = s[1] - mz * s[4];
-            const double irz = fast_recip(rz), alpha = rz * iden;
-            const double beta = (s[1] + alpha * (alpha * s[3] - 2.0 * s[2])) * irz;
+            const double alpha = quotient(rz, den, fast_recip(den));
+            const double beta = quotient(s[1] + alpha * (alpha * s[3] - 2.0 * s[2]), rz, fast_recip(rz));
             int cmd = kStep;
             if (!ok) {
                 cmd = kFail;

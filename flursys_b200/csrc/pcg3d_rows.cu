@@ -539,9 +539,8 @@ __device__ __forceinline__ bool rows_solve(const RowsArgs &a, typename RowsGroup
         lap(t_op);
         const bool ok = grp.lead(s, linf, true, face_bytes, [] {});
         if (tid < 32) {  // warp 0: the step's scalars, and the verdict on the current iterate
-            const double den = s[0], iden = fast_recip(den), rz = s[1];
-            const double irz = fast_recip(rz), alpha = rz * iden;
-            const double beta = (rz + alpha * (alpha * s[3] - 2.0 * s[2])) * irz;
+            const double den = s[0], rz = s[1], alpha = quotient(rz, den, fast_recip(den));
+            const double beta = quotient(rz + alpha * (alpha * s[3] - 2.0 * s[2]), rz, fast_recip(rz));
             int cmd = kStep;
             if (!ok) {
                 cmd = kFail;

@@ -142,13 +142,6 @@ __host__ __device__ __forceinline__ size_t sor_smem(int nx, int ny, int planes, 
     return 8 * hp * (5 * (size_t)planes + (cluster ? 6 : 4));
 }
 
-// a / diag with inv = 1 / diag at hand: the quotient's remainder corrects it
-// once, which gives the correctly rounded quotient but for rare cases.
-__device__ __forceinline__ double quotient(double a, double diag, double inv) {
-    const double q = a * inv;
-    return fma(fma(-q, diag, a), inv, q);
-}
-
 template <bool CLUSTER, typename Group>
 __device__ __forceinline__ bool sor3d_solve(const SorArgs &a, Group &grp, char *dyn) {
     const int nx = a.nx, ny = a.ny, nz = a.nz, tid = threadIdx.x, h = half_row(nx), hp = h * ny;
@@ -267,7 +260,7 @@ __device__ __forceinline__ bool sor3d_solve(const SorArgs &a, Group &grp, char *
             if (i + j + k0 + kk > 0) {
                 const double sum = nbs(0, kk, j, m, o, pc);
                 mx = fmax(mx, fabs((sum - diag * pc) - R[0][o]));
-                val = pc + a.omega * (quotient(sum - R[0][o], diag, inv) - pc);
+                val = pc + a.omega * (rounded_quotient(sum - R[0][o], diag, inv) - pc);
             }
             next_even[o] = val;
             if (more) send(0, kk, j, m, val);
@@ -292,7 +285,7 @@ __device__ __forceinline__ bool sor3d_solve(const SorArgs &a, Group &grp, char *
             const int k = k0 + kk;
             if (2 * m + ((1 + j + k) & 1) >= nx) return;
             const double pc = P[1][o];
-            const double val = pc + a.omega * (quotient(nbs(1, kk, j, m, o, pc) - R[1][o], diag, inv) - pc);
+            const double val = pc + a.omega * (rounded_quotient(nbs(1, kk, j, m, o, pc) - R[1][o], diag, inv) - pc);
             P[1][o] = val;
             send(1, kk, j, m, val);
         });
