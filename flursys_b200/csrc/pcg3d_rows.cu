@@ -748,10 +748,11 @@ bool choose_rows(Pcg3dRowsPlan &plan, int sms, bool may_cluster, bool may_grid) 
 
 bool pcg3d_rows_plan(Pcg3dRowsPlan &plan, const Pcg3dArgs &args, int precision, int device) {
     plan = Pcg3dRowsPlan{};
-    // FLURSYS_PCG_RESIDENT: 0, 2 and "stream" ask for other forms, "grid" for
-    // no cluster
+    // FLURSYS_PCG_RESIDENT: 0, 2, "tiles" and "stream" ask for other forms,
+    // "grid" for no cluster
     const char *env = std::getenv("FLURSYS_PCG_RESIDENT");
-    if (env && (std::strcmp(env, "0") == 0 || std::strcmp(env, "2") == 0 || std::strcmp(env, "stream") == 0)) return false;
+    for (const char *other : {"0", "2", "tiles", "stream"})
+        if (env && std::strcmp(env, other) == 0) return false;
     if (args.nz < 2) return false;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return false;

@@ -1803,8 +1803,8 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
     //   MIXED 22 | graph 60, 112^3 F64 22 | 43, 200^3 F64 124 | 184), MIXED up
     //   to 3.2 million cells (see there);
     // - the rest (rows above about 700 cells, larger MIXED grids): the graph.
-    // FLURSYS_PCG_RESIDENT=0 keeps the graph, =2 the tiles, =stream the
-    // streaming form.
+    // FLURSYS_PCG_RESIDENT=0 keeps the graph, =tiles the tiles, =2 those with
+    // two reductions per iteration, =stream the streaming form.
     if (!a.cg1 && plan.host_iterations == 0) {
         auto *rp = new Pcg3dRowsPlan();
         if (pcg3d_rows_plan(*rp, args, precision, device)) plan.rows = rp;

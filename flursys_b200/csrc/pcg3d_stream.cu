@@ -690,7 +690,7 @@ bool choose_stream(Pcg3dStreamPlan &plan, int most) {
 bool pcg3d_stream_plan(Pcg3dStreamPlan &plan, const Pcg3dArgs &args, int precision, int device) {
     plan = Pcg3dStreamPlan{};
     const char *env = std::getenv("FLURSYS_PCG_RESIDENT");
-    if (env && (std::strcmp(env, "0") == 0 || std::strcmp(env, "2") == 0)) return false;
+    if (env && (std::strcmp(env, "0") == 0 || std::strcmp(env, "2") == 0 || std::strcmp(env, "tiles") == 0)) return false;
     int sms = 0, per_sm = 0;
     if (args.nx < 2 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return false;
     StreamArgs &a = plan.args;
