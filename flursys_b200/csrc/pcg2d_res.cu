@@ -905,11 +905,14 @@ cudaError_t pcg2d_res_plan(Pcg2dResPlan &plan, int nx, int ny, bool plain, int p
         plan = Pcg2dResPlan{};
         return cudaSuccess;
     }
-    e = cudaMalloc(&plan.records, bytes);
-    if (e == cudaSuccess) e = cudaMemset(plan.records, 0, bytes);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // solves run on streams that do not wait for this one
-    plan.enabled = e == cudaSuccess;
-    return e;
+    if (cudaMalloc(&plan.records, bytes) != cudaSuccess || cudaMemset(plan.records, 0, bytes) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess) {  // solves run on streams that do not wait for this one
+        pcg2d_res_destroy(plan);  // no room: the streaming kernel serves the solve
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    plan.enabled = true;
+    return cudaSuccess;
 }
 
 void pcg2d_res_destroy(Pcg2dResPlan &plan) {

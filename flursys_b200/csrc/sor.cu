@@ -393,11 +393,14 @@ cudaError_t sor3d_plan(Sor3dPlan &plan, int nx, int ny, int nz, int device) {
         return cudaSuccess;
     }
     const size_t bytes = sizeof(RedRecord) * 2 * ng * (kRedSlots + 2 * (size_t)half_row(nx) * ny);
-    e = cudaMalloc(&plan.records, bytes);
-    if (e == cudaSuccess) e = cudaMemset(plan.records, 0, bytes);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // solves run on streams that do not wait for this one
-    if (e == cudaSuccess) plan.blocks = ng;
-    return e;
+    if (cudaMalloc(&plan.records, bytes) != cudaSuccess || cudaMemset(plan.records, 0, bytes) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess) {  // solves run on streams that do not wait for this one
+        sor3d_destroy(plan);  // no room: the streaming kernel serves the solve
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    plan.blocks = ng;
+    return cudaSuccess;
 }
 
 void sor3d_destroy(Sor3dPlan &plan) {
