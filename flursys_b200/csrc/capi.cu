@@ -226,15 +226,20 @@ cudaError_t PcgWorkspace::allocate3d(int nx, int ny, int nz, int prec, int devic
     return e;
 }
 
+void PcgWorkspace::free_vectors() {
+    cudaFree(r); cudaFree(d0); cudaFree(d1); cudaFree(q); cudaFree(dx);
+    r = d0 = d1 = q = nullptr; dx = nullptr;
+}
+
 void PcgWorkspace::free_all() {
+    free_vectors();
     cudaFree(row_class);
     row_class = nullptr;
     cudaFree(r_z);
     r_z = nullptr;
-    cudaFree(r); cudaFree(d0); cudaFree(d1); cudaFree(q); cudaFree(dx);
     cudaFree(partials); cudaFree(barrier); cudaFree(result);
     if (h_result) cudaFreeHost(h_result);
-    r = d0 = d1 = q = nullptr; dx = nullptr; partials = nullptr; barrier = nullptr; result = nullptr;
+    partials = nullptr; barrier = nullptr; result = nullptr;
     h_result = nullptr;
 }
 

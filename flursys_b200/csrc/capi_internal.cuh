@@ -30,6 +30,8 @@ struct PcgWorkspace {
     cudaError_t allocate(long long n, int precision, int device, int dim);
     // 3D pressure solves also need the per-row boundary class table.
     cudaError_t allocate3d(int nx, int ny, int nz, int precision, int device, cudaStream_t stream);
+    // Frees the vectors of a 3D solve that runs on others.
+    void free_vectors();
     void free_all();
 };
 

@@ -87,6 +87,8 @@ static int32_t init3d(FlursysCudaHandle *h) {
         e = pcg3d_seq_plan(h->seq, a, c.precision, h->device);
         if (e == cudaSuccess) e = cudaMallocHost(&h->h_seq, sizeof(CgSeqState));
         if (e != cudaSuccess) return set_cuda_error(&h->err, e, "building the pressure-solve graph");
+        // these forms hold their own vectors (streaming) or none (rows)
+        if (h->seq.rows || h->seq.stream) h->pcg.free_vectors();
     }
     return FLURSYS_OK;
 }

@@ -66,3 +66,22 @@ def test_no_room_for_the_resident_records(oracle, monkeypatch, case):
     del filler
     torch.cuda.empty_cache()
     assert np.array_equal(p, ref)  # the streaming kernel's result
+
+
+@pytest.mark.parametrize("form,precision,vectors", [
+    ("stream", _abi.PRECISION_F64, 1 * 8),    # the graph holds r, two d and q; this form two r, two d and the increment
+    ("stream", _abi.PRECISION_MIXED, 0),      # the graph has the increment too
+    ("grid", _abi.PRECISION_MIXED, -5 * 4),   # rows: all on the chip
+])
+def test_a_form_with_its_own_vectors_does_not_hold_the_graphs(oracle, monkeypatch, form, precision, vectors):
+    from .test_gpu_cavity3d import cfg3d
+    shape = (160, 160, 160) if form == "stream" else (128, 128, 128)
+    cfg = cfg3d(oracle, *shape, precision=precision)
+    cfg.pressure_max_iters = 20
+    used = {}
+    for env in ("0", form):
+        monkeypatch.setenv("FLURSYS_PCG_RESIDENT", env)
+        _footprint(cfg)
+        used[env] = _footprint(cfg)
+    # records, faces and the rounding of allocations to 2 MB: a few MB
+    assert used[form] - used["0"] <= vectors * np.prod(shape) + 16 * MB
