@@ -197,7 +197,16 @@ int32_t run_pcg3d(PcgWorkspace &ws, int nx, int ny, int nz, double dx, double dy
     return FLURSYS_OK;
 }
 
-cudaError_t PcgWorkspace::allocate(long long n, int precision, int device, int dim) {
+cudaError_t PcgWorkspace::allocate_vectors(long long n) {
+    const size_t vb = precision == FLURSYS_PRECISION_MIXED ? sizeof(float) : sizeof(double);
+    cudaError_t e = cudaSuccess;
+    for (void **v : {&r, &d0, &d1, &q})
+        if (e == cudaSuccess) e = cudaMalloc(v, vb * n);
+    if (e == cudaSuccess && precision == FLURSYS_PRECISION_MIXED) e = cudaMalloc(&dx, sizeof(float) * n);
+    return e;
+}
+
+cudaError_t PcgWorkspace::allocate(long long n, int precision, int device, int dim, bool vectors) {
     free_all();
     this->precision = precision;
     int maxgrid = 0;
@@ -206,13 +215,8 @@ cudaError_t PcgWorkspace::allocate(long long n, int precision, int device, int d
     const int bs = dim == 3 ? pcg3d_block_size() : pcg2d_block_size();
     long long want = (n + (long long)bs * 4 - 1) / ((long long)bs * 4);  // >= 4 cells per thread
     grid = (int)std::max(1LL, std::min((long long)maxgrid, want));
-    const size_t vb = precision == FLURSYS_PRECISION_MIXED ? sizeof(float) : sizeof(double);
     const int np = dim == 3 ? pcg3d_num_partials() : pcg2d_num_partials();
-    if ((e = cudaMalloc(&r, vb * n)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&d0, vb * n)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&d1, vb * n)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&q, vb * n)) != cudaSuccess) return e;
-    if (precision == FLURSYS_PRECISION_MIXED && (e = cudaMalloc(&dx, sizeof(float) * n)) != cudaSuccess) return e;
+    if (vectors && (e = allocate_vectors(n)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&partials, sizeof(double) * (size_t)np * grid)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&barrier, sizeof(GridBarrier))) != cudaSuccess) return e;
     if ((e = cudaMalloc(&result, sizeof(PcgResultDev))) != cudaSuccess) return e;
@@ -220,26 +224,21 @@ cudaError_t PcgWorkspace::allocate(long long n, int precision, int device, int d
     return cudaSuccess;
 }
 
-cudaError_t PcgWorkspace::allocate3d(int nx, int ny, int nz, int prec, int device, cudaStream_t stream) {
-    cudaError_t e = allocate((long long)nx * ny * nz, prec, device, 3);
+cudaError_t PcgWorkspace::allocate3d(int nx, int ny, int nz, int prec, int device, cudaStream_t stream, bool vectors) {
+    cudaError_t e = allocate((long long)nx * ny * nz, prec, device, 3, vectors);
     if (e == cudaSuccess) e = pcg3d_make_row_class(ny, nz, &row_class, stream);
     return e;
 }
 
-void PcgWorkspace::free_vectors() {
-    cudaFree(r); cudaFree(d0); cudaFree(d1); cudaFree(q); cudaFree(dx);
-    r = d0 = d1 = q = nullptr; dx = nullptr;
-}
-
 void PcgWorkspace::free_all() {
-    free_vectors();
     cudaFree(row_class);
     row_class = nullptr;
     cudaFree(r_z);
     r_z = nullptr;
+    cudaFree(r); cudaFree(d0); cudaFree(d1); cudaFree(q); cudaFree(dx);
     cudaFree(partials); cudaFree(barrier); cudaFree(result);
     if (h_result) cudaFreeHost(h_result);
-    partials = nullptr; barrier = nullptr; result = nullptr;
+    r = d0 = d1 = q = nullptr; dx = nullptr; partials = nullptr; barrier = nullptr; result = nullptr;
     h_result = nullptr;
 }
 

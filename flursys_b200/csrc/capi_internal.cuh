@@ -27,11 +27,11 @@ struct PcgWorkspace {
     PcgResultDev *h_result = nullptr;  // pinned host copy
     unsigned char *row_class = nullptr;  // 3D: per-row boundary class
     int precision = 0;
-    cudaError_t allocate(long long n, int precision, int device, int dim);
-    // 3D pressure solves also need the per-row boundary class table.
-    cudaError_t allocate3d(int nx, int ny, int nz, int precision, int device, cudaStream_t stream);
-    // Frees the vectors of a 3D solve that runs on others.
-    void free_vectors();
+    cudaError_t allocate(long long n, int precision, int device, int dim, bool vectors = true);
+    // 3D pressure solves also need the per-row boundary class table. Without
+    // `vectors`, r, d0, d1, q and dx are left to allocate_vectors().
+    cudaError_t allocate3d(int nx, int ny, int nz, int precision, int device, cudaStream_t stream, bool vectors = true);
+    cudaError_t allocate_vectors(long long n);
     void free_all();
 };
 

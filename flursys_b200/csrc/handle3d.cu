@@ -53,7 +53,13 @@ static int32_t init3d(FlursysCudaHandle *h) {
     }
     cudaError_t e = cudaMalloc(&h->diag3, sizeof(Diag3Dev));
     if (e == cudaSuccess) e = cudaMallocHost(&h->h_diag3, sizeof(Diag3Dev));
-    if (e == cudaSuccess) e = h->pcg.allocate3d((int)c.nx, (int)c.ny, (int)c.nz, c.precision, h->device, h->stream);
+    // FLURSYS_PCG_VARIANT=persistent selects the single cooperative kernel; the
+    // other PCG forms allocate the vectors that they need when they are planned.
+    const char *variant = std::getenv("FLURSYS_PCG_VARIANT");
+    h->use_seq = c.pressure_solver != FLURSYS_PRESSURE_SOR && c.pressure_solver != FLURSYS_PRESSURE_FCG &&
+                 !(variant && std::strcmp(variant, "persistent") == 0);
+    if (e == cudaSuccess)
+        e = h->pcg.allocate3d((int)c.nx, (int)c.ny, (int)c.nz, c.precision, h->device, h->stream, !h->use_seq);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return set_cuda_error(&h->err, e, "allocating 3D solver workspace");
     if (c.pressure_solver == FLURSYS_PRESSURE_FCG) {
@@ -75,20 +81,18 @@ static int32_t init3d(FlursysCudaHandle *h) {
         e = sor3d_plan(h->sor, s.nx, s.ny, s.nz, h->device);
         if (e != cudaSuccess) return set_cuda_error(&h->err, e, "planning the SOR solve");
     }
-    // The graph-driven PCG is the default; FLURSYS_PCG_VARIANT=persistent
-    // selects the single cooperative kernel instead.
-    const char *variant = std::getenv("FLURSYS_PCG_VARIANT");
-    h->use_seq = c.pressure_solver != FLURSYS_PRESSURE_SOR && !(variant && std::strcmp(variant, "persistent") == 0);
     if (h->use_seq) {
         const int rule = c.stop_rule == FLURSYS_STOP_REFERENCE_RESIDUAL ? FLURSYS_STOP_ABS_INF : c.stop_rule;
         Pcg3dArgs a = make_pcg3d_args(h->pcg, s.nx, s.ny, s.nz, s.dx, s.dy, s.dz, s.p, s.rhs, c.precision, rule,
                                       c.pressure_tolerance, c.pressure_atol, c.pressure_rtol, c.pressure_max_iters,
                                       c.residual_replacement_every);
-        e = pcg3d_seq_plan(h->seq, a, c.precision, h->device);
+        e = pcg3d_seq_plan(h->seq, a, c.precision, h->device, [&](Pcg3dArgs &args) {
+            const cudaError_t ve = h->pcg.allocate_vectors(nc);
+            args.r = h->pcg.r; args.d0 = h->pcg.d0; args.d1 = h->pcg.d1; args.q = h->pcg.q; args.dx = h->pcg.dx;
+            return ve;
+        });
         if (e == cudaSuccess) e = cudaMallocHost(&h->h_seq, sizeof(CgSeqState));
         if (e != cudaSuccess) return set_cuda_error(&h->err, e, "building the pressure-solve graph");
-        // these forms hold their own vectors (streaming) or none (rows)
-        if (h->seq.rows || h->seq.stream) h->pcg.free_vectors();
     }
     return FLURSYS_OK;
 }

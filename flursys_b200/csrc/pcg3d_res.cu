@@ -837,8 +837,7 @@ __global__ void __launch_bounds__(BLK, 1) pcg3d_res1_kernel(const __grid_constan
 
 }  // namespace
 
-bool pcg3d_res_plan(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device) {
-    plan = Pcg3dResPlan{};
+static bool res_split(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device, int &sms) {
     const char *env = std::getenv("FLURSYS_PCG_RESIDENT");
     if (env && (std::strcmp(env, "0") == 0 || std::strcmp(env, "stream") == 0)) return false;
     if (args.nz < 2) return false;
@@ -848,7 +847,6 @@ bool pcg3d_res_plan(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device) {
     a.n = a.nxy * args.nz;
     a.ntx = (a.nx + RX - 1) / RX;
     a.nty = (a.ny + RY - 1) / RY;
-    int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return false;
     const long long cols = (long long)a.ntx * a.nty;
     if (cols > sms) return false;
@@ -857,7 +855,21 @@ bool pcg3d_res_plan(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device) {
     if (a.tz > kResMaxTz) return false;
     a.ntz = (a.nz + a.tz - 1) / a.tz;
     plan.grid = (int)(cols * a.ntz);
-    if (plan.grid > kResMaxBlocks) return false;
+    return plan.grid <= kResMaxBlocks;
+}
+
+bool pcg3d_res_fits(const Pcg3dArgs &args, int device) {
+    Pcg3dResPlan plan;
+    int sms = 0;
+    return res_split(plan, args, device, sms);
+}
+
+bool pcg3d_res_plan(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device) {
+    plan = Pcg3dResPlan{};
+    int sms = 0, per_sm = 0;
+    if (!res_split(plan, args, device, sms)) return false;
+    const char *env = std::getenv("FLURSYS_PCG_RESIDENT");
+    ResArgs &a = plan.args;
     plan.smem = res_smem_bytes(a.tz);
     // one reduction per iteration for the L2 stop rule (FLURSYS_PCG_RESIDENT=2
     // keeps the two-reduction form)

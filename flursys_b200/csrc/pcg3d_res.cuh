@@ -51,6 +51,8 @@ struct Pcg3dResPlan {
 // args.q are the FP32 face-exchange buffers); false when the grid does not fit one tile per
 // SM, the device cannot hold a tile, or FLURSYS_PCG_RESIDENT asks for another form.
 bool pcg3d_res_plan(Pcg3dResPlan &plan, const Pcg3dArgs &args, int device);
+// Whether the grid fits, by its size and the environment alone (no vectors needed).
+bool pcg3d_res_fits(const Pcg3dArgs &args, int device);
 // One solve; the result is written to *state (CgSeqState fields error,
 // status, iterations, initial, initial_l2, residual, true_l2, device_error).
 cudaError_t pcg3d_res_launch(const Pcg3dResPlan &plan, CgSeqState *state, cudaStream_t stream);

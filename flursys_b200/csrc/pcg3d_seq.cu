@@ -1693,7 +1693,8 @@ cudaError_t build_cg1(Pcg3dSeqPlan &plan, SeqArgs &a, const Cg1Maps &maps) {
 
 }  // namespace
 
-cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precision, int device) {
+cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, Pcg3dArgs args, int precision, int device,
+                           const std::function<cudaError_t(Pcg3dArgs &)> &vectors) {
     pcg3d_seq_destroy(plan);
     SeqArgs a{};
     SeqGeo &g = a.g;
@@ -1751,7 +1752,6 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
     a.nblocks_point = std::max(1, std::min(sms * point_per_sm, (g.n / 4 + kBlock - 1) / kBlock));
     a.x = args.x;
     a.rhs = args.rhs;
-    a.r = args.r; a.d0 = args.d0; a.d1 = args.d1; a.q = args.q; a.dx = args.dx;
     a.row_class = args.row_class;
     a.stop_rule = args.stop_rule;
     a.tol = args.tol; a.atol = args.atol; a.rtol = args.rtol;
@@ -1811,7 +1811,11 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
         else delete rp;
         cudaGetLastError();  // a declined plan leaves no sticky error behind
     }
-    if (!plan.rows && precision == FLURSYS_PRECISION_MIXED && !a.cg1 && plan.host_iterations == 0) {
+    bool have_vectors = false;
+    if (!plan.rows && precision == FLURSYS_PRECISION_MIXED && !a.cg1 && plan.host_iterations == 0 && pcg3d_res_fits(args, device)) {
+        e = vectors(args);
+        if (e != cudaSuccess) return e;
+        have_vectors = true;
         auto *rp = new Pcg3dResPlan();
         if (pcg3d_res_plan(*rp, args, device)) plan.resident = rp;
         else delete rp;
@@ -1823,6 +1827,11 @@ cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precis
         else delete sp;
         cudaGetLastError();
     }
+    if (!plan.rows && !plan.resident && !plan.stream && !have_vectors) {
+        e = vectors(args);
+        if (e != cudaSuccess) return e;
+    }
+    a.r = args.r; a.d0 = args.d0; a.d1 = args.d1; a.q = args.q; a.dx = args.dx;
     Cg1Maps maps{};
     if (a.cg1) {
         a.cr[0] = static_cast<float *>(args.r);

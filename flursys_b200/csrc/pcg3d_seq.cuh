@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
+
 #include "pcg3d.cuh"
 
 namespace flursys {
@@ -40,9 +42,12 @@ struct Pcg3dSeqPlan {
     void *cg1_maps = nullptr;   // tensor maps of the single-reduction step kernel
 };
 
-// Builds and instantiates the solve graph for fixed buffers (args as for
-// pcg3d_launch, barrier/result/partials unused).
-cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, const Pcg3dArgs &args, int precision, int device);
+// Chooses the form of the solve for fixed buffers (args as for pcg3d_launch,
+// barrier/result/partials unused) and sets it up; the graph is built where no
+// other form serves the grid. `vectors` fills args.r, d0, d1, q and dx; it is
+// called for a form that works on them (the tiles, the graph).
+cudaError_t pcg3d_seq_plan(Pcg3dSeqPlan &plan, Pcg3dArgs args, int precision, int device,
+                           const std::function<cudaError_t(Pcg3dArgs &)> &vectors);
 cudaError_t pcg3d_seq_launch(const Pcg3dSeqPlan &plan, cudaStream_t stream);
 void pcg3d_seq_destroy(Pcg3dSeqPlan &plan);
 cudaError_t pcg3d_seq_run_host(const Pcg3dSeqPlan &plan, cudaStream_t stream);
