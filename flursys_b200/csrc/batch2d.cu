@@ -452,16 +452,17 @@ float time_ms(FlursysBatchHandle *h, int reps, F fn, cudaError_t *e) {
 // grid), the cooperative launch runs after the queue, and an instance that
 // would share it costs little there: the index in `order` (largest first) from
 // which on instances are queued so that both launches together take least time.
-// A queued iteration takes about 2.9 us + 42 ps per cell on its cluster; the
-// cooperative launch takes 15.8 (F64: 12.2) us for each iteration of its
+// A queued iteration takes about 3.0 (F64: 2.9) us and 47 (42) ps per cell on its
+// cluster; the cooperative launch takes 15.8 (12.2) us for each iteration of its
 // longest instance and 14.2 (19) ps for each cell and iteration of any. Per
 // step in MIXED, all that fit queued and as chosen here: 512^2 + 520^2 63 and
 // 46 ms, 512^2 + 600^2 76 and 53, eight 64^2 + 600^2 52 and 49, three 448^2 +
-// three 600^2 89 and 81. (A batch that fits the queue as a whole is 1.5 to 3.9
+// three 600^2 89 and 81. (A batch that fits the queue as a whole is 1.3 to 3.9
 // times faster there at any count.)
 int queue_from(const FlursysBatchHandle *h, const std::vector<int> &order) {
     const bool mixed = h->precision == FLURSYS_PRECISION_MIXED;
     const double base = mixed ? 15.8 : 12.2, per_cell = mixed ? 14.2e-6 : 19.0e-6;
+    const double queue_base = mixed ? 3.0 : 2.9, queue_per_cell = mixed ? 47.0e-6 : 42.0e-6;
     // iterations grow with the longer side; SOR needs several times as many
     auto its = [&](int i) { return double(std::max(h->nx[i], h->ny[i])) * (h->h_pin[i].solver == FLURSYS_PRESSURE_SOR ? 8.0 : 1.0); };
     auto cells = [&](int i) { return double(h->h_ctl[i].cells); };
@@ -476,7 +477,7 @@ int queue_from(const FlursysBatchHandle *h, const std::vector<int> &order) {
     for (int first = 0; first <= (int)order.size(); ++first) {
         std::vector<double> busy(h->queue.clusters, 0.0);
         for (int k = first; k < (int)order.size(); ++k)
-            *std::min_element(busy.begin(), busy.end()) += its(order[k]) * (2.9 + 42.0e-6 * cells(order[k]));
+            *std::min_element(busy.begin(), busy.end()) += its(order[k]) * (queue_base + queue_per_cell * cells(order[k]));
         const double t = *std::max_element(busy.begin(), busy.end()) + base * longest + per_cell * work;
         if (first == 0 || t < best) {
             best = t;

@@ -7,14 +7,15 @@
 // warp's reads do not conflict), and so do d, r and the inverse diagonal of
 // every column that the rows can reach (own rows and a band on each side). An
 // iteration is one pass q = A d over the own rows, which also forms the
-// products d.q, r.Mr, q.Mr, q.Mq and r.r, one grid-wide sum (gridreduce.cuh), and one pass that updates x, r and d = M r +
-// beta d on the own rows and, from the neighbours' q, on the band, with the
-// owners' arithmetic. beta uses r.Mr - 2 alpha q.Mr + alpha^2 q.Mq of the
+// products d.q, r.Mr, q.Mr, q.Mq and r.r, one grid-wide sum (gridreduce.cuh),
+// and one pass that updates x, r and d = M r + beta d on the own rows and, from
+// the neighbours' q, on the band, with the owners' arithmetic. beta uses r.Mr - 2 alpha q.Mr + alpha^2 q.Mq of the
 // directly summed products. ||r|| is tested where r.r is summed, one pass
 // after its update; row sums keep the CSR order.
 //
-// What bounds it: the round through L2 (about 3 us) and the passes' shared
-// memory traffic. Per iteration, against the cooperative kernel with two
+// What bounds it: the round through L2 (about 3 us) and the latency of the
+// passes' gathers (262144 rows with a band of 1024: shared memory 47% busy, issue
+// slots 37%). Per iteration, against the cooperative kernel with two
 // barriers (csr.cu): 32768 rows with a band of 64 17 -> 4.1 us, 262144 rows
 // with a band of 1024 18.5 -> 5.4 us. (With q as plain stores behind the
 // round's fences instead of records: 7.0 and 6.5 us.)

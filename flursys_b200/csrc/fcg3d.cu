@@ -174,8 +174,9 @@ __global__ void __launch_bounds__(kPw) fcg_shift(double *x, const FcgScalars *sc
 // instead of stored. The operator arithmetic per cell is that of apply7, in
 // its order, with weight 0 where there is no neighbour.
 //
-// What bounds them: HBM (8, 12 and 12 bytes per cell; a thread per cell, with
-// its neighbour tests, was bound by issue). Per pass on 256^3, before and
+// What bounds them: HBM (operator 12 bytes per cell, pre-smoothing 8, post-
+// smoothing 12: 31, 21 and 31 us on 256^3 at the copy rate; a thread per cell,
+// with its neighbour tests, was bound by issue). Per pass there, before and
 // after: operator 56 and 44 us, pre-smoothing 69 and 30, post-smoothing 73 and 44.
 struct March {
     int nvec, kz;  // vectors of a row, planes of a block

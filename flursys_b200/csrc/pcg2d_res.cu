@@ -32,8 +32,10 @@
 // 331 took 5.5 us instead of 5.9, and a solve to 1e-12 2761 of them instead of
 // 2563.)
 //
-// What bounds it: on small grids latency (the block reduction, the exchange,
-// the scalars' chain), on large ones instruction issue. A lane takes 16 bytes
+// What bounds it: latency. On small grids that of the block reduction, the
+// exchange and the scalars' chain; on large ones also the passes', two warps per
+// scheduler (four in the queue) that keep issue slots 26% (52%) busy and wait on
+// shared memory, conversions and barriers. A lane takes 16 bytes
 // of a row at a time, and without solid or outlet cells the direction's ghost
 // cells hold the wall cell's own value, so that the operator has no boundary
 // case (a pass that derived each cell's position and couplings spent 240

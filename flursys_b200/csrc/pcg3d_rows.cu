@@ -19,13 +19,20 @@
 // MIXED), r and x in registers. Cells per block and faces decide the split:
 // see pcg3d_rows_plan().
 //
-// What bounds it: on small grids the round (partials and faces through L2 or,
-// in a cluster, through distributed shared memory), on large ones shared-memory
-// bandwidth, the FP32 -> FP64 conversions of the inner products and instruction
-// issue; DRAM sees the pressure only at the residual replacements. Per
-// iteration, against the graph-driven form: 75 x 62 x 51 F64 22.5 -> 6.1 us,
-// 64^3 MIXED 20 -> 4.6, 100^3 F64 39 -> 13.6, 128^3 MIXED 30 -> 16.3 (the
-// tile-resident form of pcg3d_res.cu: 20).
+// What bounds it: latency. On small grids the round (partials and faces through
+// L2 or, in a cluster, through distributed shared memory); on large ones four
+// warps per scheduler that wait on shared memory, L2, their own chains and the
+// block's barriers: at 128^3 in MIXED issue slots are 43% busy, shared memory
+// 35%, the conversions' unit 10%, FP64 6%. DRAM sees the pressure only at the
+// residual replacements. Per iteration, against the graph-driven form:
+// 75 x 62 x 51 F64 22.5 -> 6.1 us, 64^3 MIXED 20 -> 4.6, 100^3 F64 39 -> 13.6,
+// 128^3 MIXED 30 -> 16.3 (the tile-resident form of pcg3d_res.cu: 20).
+//
+// MIXED applies alpha and beta rounded to FP32, the same to x and r, as the tile
+// form does (the graph rounds beta alone). With alpha in FP64 128^3 took 15%
+// longer at the same errors against 64 bits: on average 6% of the graph's and the
+// tiles' in the pressure and 75% in the velocities (their operator is a sum that
+// does not annihilate a constant exactly).
 #include <cuda_runtime.h>
 
 #include <algorithm>

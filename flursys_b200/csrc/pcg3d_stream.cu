@@ -24,10 +24,17 @@
 // What bounds it: the latency of one plane's chain beside DRAM. 256^3 in MIXED
 // moves 403 MB per iteration, 62 us at the copy rate; a pass that only moves
 // them takes 74 us with its sum, the solve 103 us (two launches per iteration:
-// 139 to 147). One vector column per thread fills the registers of four warps
+// 139 to 147). On 160 x 140 x 120, which lies in L2, issue slots are 49% busy
+// and shared memory 34%; the warps wait at the plane's barrier and on their
+// loads. One vector column per thread fills the registers of four warps
 // per scheduler; two spill some thirty. Per iteration, against the graph:
 // 160^3 MIXED 50 -> 30 us, 300 x 200 x 150 MIXED 95 -> 84, 112^3 F64 43 -> 22,
 // 200^3 F64 184 -> 124.
+//
+// MIXED applies alpha and beta rounded to FP32, the same to x and r (the graph
+// rounds beta alone; see pcg3d_rows.cu): with alpha in FP64 160 x 140 x 120 took
+// 29.1 us instead of 26.5, and the errors against 64 bits are half the graph's in
+// the velocities, a twentieth in the pressure, either way.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -704,11 +711,12 @@ bool pcg3d_stream_plan(Pcg3dStreamPlan &plan, const Pcg3dArgs &args, int precisi
     a.replace_every = args.replace_every > 0 ? args.replace_every : 50;
     const bool mixed = precision == FLURSYS_PRECISION_MIXED;
     const int most = std::min(sms, 160);
-    // A MIXED solve of a larger grid to 1e-12 ends with an error of the
-    // pressure's constant part (the pin's tiny eigenvalue) of 1e-9 and more,
-    // in which forms that round differently differ as much (256^3: 1e-10 to
-    // 2.4e-9 of the pressure, 144^3: at most 8e-10; velocities 1e-13): there the
-    // graph stays, and its results with it.
+    // The limit keeps what this form and the graph return within 1e-9 of each
+    // other (2-norm of the pressure), so that one may stand for the other in
+    // a running program; it is not a limit of speed. A MIXED solve by the graph
+    // to 1e-12 ends with an error of the pressure's constant part (the pin's
+    // tiny eigenvalue) that grows with the grid, and the two forms differ by
+    // it: 256^3 1e-10 to 2.4e-9, 144^3 at most 8e-10 (velocities 1e-13).
     if (mixed && !(env && std::strcmp(env, "stream") == 0) && (long long)args.nx * args.ny * args.nz > 3'200'000LL) return false;
     if (!(mixed ? choose_stream<float>(plan, most) : choose_stream<double>(plan, most))) return false;
     const size_t bytes = (mixed ? 4 * (size_t)row_pitch<float>(a.nx) : 8 * (size_t)row_pitch<double>(a.nx)) * a.ny * a.nz;
