@@ -572,12 +572,17 @@ __device__ __forceinline__ bool rows_solve(const RowsArgs &a, typename RowsGroup
                 cmd = kStop;
             }
             if (cmd == kStep) {
-                iterations = it + 1;
-                if (!(fabs(den) >= 1.0e-30 && fabs(den) <= 1.7976931348623157e308) || !isfinite(alpha)) {
-                    error = FLURSYS_ERR_BREAKDOWN;
-                    cmd = kStop;
+                const bool sound = fabs(den) >= 1.0e-30 && fabs(den) <= 1.7976931348623157e308 && isfinite(alpha);
+                if (MIXED && !sound && since > 0) {
+                    cmd = kRefresh;  // the FP32 recurrence has run out before its replacement was due
+                } else {
+                    iterations = it + 1;
+                    if (!sound) {
+                        error = FLURSYS_ERR_BREAKDOWN;
+                        cmd = kStop;
+                    }
+                    rz_old = rz;
                 }
-                rz_old = rz;
             }
             if (tid == 0) {
                 sc.alpha = V(alpha);
