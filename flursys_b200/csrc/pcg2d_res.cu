@@ -879,9 +879,17 @@ cudaError_t pcg2d_res_plan(Pcg2dResPlan &plan, int nx, int ny, bool plain, int p
         }
         return false;
     };
+    // Rows of a few vectors leave most lanes of a warp idle, and many of them
+    // make a block's passes long: a piece (32 vectors' room) per warp takes 0.85
+    // us of an iteration in F64, 1.25 in MIXED. A cluster with more than six
+    // leaves the solve to the grid (4 x 5000 F64 18.5 us, grid 10.4), and a grid
+    // whose pieces cost more than the streaming kernel's iteration leaves it
+    // to that (4 x 100000 MIXED 56.3 us, streaming 26.5; 6 x 100000 F64 41.3 and
+    // 33.4; but 16 x 40000 MIXED 26.0 and 34.5).
+    auto pieces = [&]() { return pieces_of(precision, plan.variant, (ny + plan.nblocks - 1) / plan.nblocks, nx); };
     if (may_cluster && n <= cluster_cells) {
         const int nb = (int)std::max(1LL, std::min<long long>(kMaxCluster, (n + 255) / 256));
-        if (choose(true, nb)) {
+        if (choose(true, nb) && pieces() <= 6) {
             const int nb = plan.nblocks;
             const void *fn = res_fn<true>(precision, plan.variant);
             cudaLaunchAttribute attr[1];
@@ -896,7 +904,8 @@ cudaError_t pcg2d_res_plan(Pcg2dResPlan &plan, int nx, int ny, bool plain, int p
         }
     }
     const int nb = (int)std::max(1LL, std::min<long long>(std::min(sms, 160), (n + 511) / 512));
-    if (!choose(false, nb)) {
+    const double piece_us = precision == FLURSYS_PRECISION_MIXED ? 1.25 : 0.85;
+    if (!choose(false, nb) || 3.5 + piece_us * pieces() > 11.0 + 36.0e-6 * double(n)) {
         plan = Pcg2dResPlan{};
         return cudaSuccess;
     }
