@@ -99,11 +99,11 @@ __host__ __device__ __forceinline__ int op_elems(int op, int nx, int ny) {
 // Pressure blocks in proportion to cells x iterations of the previous step
 // (an estimate of 4 sqrt(cells) before the first one); one block at least,
 // and no more than one per kBlk cells. Run by one thread.
-__device__ void share_pressure_blocks(const BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_blocks) {
+__device__ void share_pressure_blocks(const BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_blocks, int queued) {
     double wsum = 0.0;
     int nact = 0;
     for (int t = 0; t < n; ++t) {
-        if (!ctl[t].active || pin[t].resident) continue;
+        if (!ctl[t].active || (queued && pin[t].resident)) continue;
         const double cells = double(ctl[t].cells);
         const double its = ctl[t].last_iters > 0 ? double(ctl[t].last_iters) : 4.0 * sqrt(cells);
         wsum += cells * its;
@@ -113,8 +113,9 @@ __device__ void share_pressure_blocks(const BatchCtl *ctl, Pcg2dInstance *pin, i
     int b0 = 0;
     for (int t = 0; t < n; ++t) {
         pin[t].block0 = b0;
-        if (pin[t].resident) pin[t].resident = ctl[t].active ? 1 : -1;
-        if (!ctl[t].active || pin[t].resident) {
+        const bool resident = queued && pin[t].resident;
+        if (resident) pin[t].resident = ctl[t].active ? 1 : -1;
+        if (!ctl[t].active || resident) {
             pin[t].nblocks = 0;
             continue;
         }
@@ -135,13 +136,13 @@ __device__ __forceinline__ void reset_barrier(GridBarrier *b) {
 }
 
 // Pressure launch set-up alone (tuning runs): barriers and block shares.
-__global__ void batch_prepare_pressure(const BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_blocks) {
+__global__ void batch_prepare_pressure(const BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_blocks, int queued) {
     for (int t = threadIdx.x; t < n; t += blockDim.x) reset_barrier(pin[t].barrier);
     __syncthreads();
-    if (threadIdx.x == 0) share_pressure_blocks(ctl, pin, n, total_blocks);
+    if (threadIdx.x == 0) share_pressure_blocks(ctl, pin, n, total_blocks, queued);
 }
 
-__global__ void batch_begin(BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_blocks, unsigned *queue_next) {
+__global__ void batch_begin(BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_blocks, int queued, unsigned *queue_next) {
     if (threadIdx.x == 0) *queue_next = 0u;
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         BatchCtl &c = ctl[t];
@@ -178,7 +179,7 @@ __global__ void batch_begin(BatchCtl *ctl, Pcg2dInstance *pin, int n, int total_
         c.step_dt = dt;
     }
     __syncthreads();
-    if (threadIdx.x == 0) share_pressure_blocks(ctl, pin, n, total_blocks);
+    if (threadIdx.x == 0) share_pressure_blocks(ctl, pin, n, total_blocks, queued);
 }
 
 template <int OP>
@@ -415,7 +416,7 @@ cudaError_t set_tiles(FlursysBatchHandle *h, int op, int elems) {
 }
 
 cudaError_t enqueue_step(FlursysBatchHandle *h, cudaStream_t st) {
-    batch_begin<<<1, kBlk, 0, st>>>(h->ctl, h->pin, h->n, h->pcg_blocks, h->queue_next);
+    batch_begin<<<1, kBlk, 0, st>>>(h->ctl, h->pin, h->n, h->pcg_blocks, h->queued, h->queue_next);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = launch_op(h, kOpPredict, st);
     if (e == cudaSuccess) e = launch_op(h, kOpBndStar, st);
@@ -448,47 +449,70 @@ float time_ms(FlursysBatchHandle *h, int reps, F fn, cudaError_t *e) {
     return ms / reps;
 }
 
-// Where a batch has instances that the queue cannot take (SOR, too large a
-// grid), the cooperative launch runs after the queue, and an instance that
-// would share it costs little there: the index in `order` (largest first) from
-// which on instances are queued so that both launches together take least time.
-// A queued iteration takes about 3.0 (F64: 2.9) us and 47 (42) ps per cell on its
-// cluster; the cooperative launch takes 15.8 (12.2) us for each iteration of its
-// longest instance and 14.2 (19) ps for each cell and iteration of any. Per
-// step in MIXED, all that fit queued and as chosen here: 512^2 + 520^2 63 and
-// 46 ms, 512^2 + 600^2 76 and 53, eight 64^2 + 600^2 52 and 49, three 448^2 +
-// three 600^2 89 and 81. (A batch that fits the queue as a whole is 1.3 to 3.9
-// times faster there at any count.)
-int queue_from(const FlursysBatchHandle *h, const std::vector<int> &order) {
+// Which of the instances that fit the queue (`order`, largest first) it takes:
+// those whose choice makes both launches, which follow one another, shortest by
+// the estimates below (us; an instance's iterations grow with its longer side,
+// SOR's sweeps are several times as many). Either the largest or the smallest
+// are left to the cooperative launch, or none, or all.
+//
+// Queue: a cluster's iterations one after another. Per iteration, MIXED (F64):
+// 64^2 3.7 (3.1), 256^2 6.0 (5.7), 512^2 15.6; rows of a few cells by pieces per
+// warp (4 x 2000 12.8 and 8.2).
+// Cooperative launch: its longest instance's two barriers per iteration and the
+// work of all, which share the chip. Per iteration in MIXED one 64^2 11.5,
+// sixteen 13, 256 of them 21; one 512^2 19.7; 32 of 256^2 43, and a third more
+// per cell where the vectors outgrow L2.
+//
+// Per step, MIXED, queue and cooperative launch: 256 instances of 32^2 16.7 and
+// 1.3 ms, 64 of 64^2 8.7 and 3.7, 48 of 128^2 12.8 and 11.7, 32 of 256^2 29 and
+// 43, 64 of 64^2 to 448^2 77 and 139; 512^2 queued and 520^2 launched 63, both
+// launched 46.
+std::vector<int> queue_of(const FlursysBatchHandle *h, const std::vector<int> &order) {
     const bool mixed = h->precision == FLURSYS_PRECISION_MIXED;
-    const double base = mixed ? 15.8 : 12.2, per_cell = mixed ? 14.2e-6 : 19.0e-6;
-    const double queue_base = mixed ? 3.0 : 2.9, queue_per_cell = mixed ? 47.0e-6 : 42.0e-6;
-    // iterations grow with the longer side; SOR needs several times as many
-    auto its = [&](int i) { return double(std::max(h->nx[i], h->ny[i])) * (h->h_pin[i].solver == FLURSYS_PRESSURE_SOR ? 8.0 : 1.0); };
-    auto cells = [&](int i) { return double(h->h_ctl[i].cells); };
-    double longest = 0.0, work = 0.0;  // of the cooperative launch
-    for (int i = 0; i < h->n; ++i)
-        if (std::find(order.begin(), order.end(), i) == order.end()) {
-            longest = std::max(longest, its(i));
-            work += cells(i) * its(i);
-        }
-    int best_first = 0;
-    double best = 0.0;
-    for (int first = 0; first <= (int)order.size(); ++first) {
-        std::vector<double> busy(h->queue.clusters, 0.0);
-        for (int k = first; k < (int)order.size(); ++k)
-            *std::min_element(busy.begin(), busy.end()) += its(order[k]) * (queue_base + queue_per_cell * cells(order[k]));
-        const double t = *std::max_element(busy.begin(), busy.end()) + base * longest + per_cell * work;
-        if (first == 0 || t < best) {
-            best = t;
-            best_first = first;
-        }
-        if (first < (int)order.size()) {
-            longest = std::max(longest, its(order[first]));
-            work += cells(order[first]) * its(order[first]);
-        }
+    struct Load {
+        double its, queued, base, work, cells;
+    };
+    std::vector<Load> load(h->n);
+    for (int i = 0; i < h->n; ++i) {
+        const double side = std::max(h->nx[i], h->ny[i]), cells = double(h->h_ctl[i].cells);
+        const bool plain = h->h_pin[i].count_fluid == h->h_ctl[i].cells;
+        Load &l = load[i];
+        l.its = side * (h->h_pin[i].solver == FLURSYS_PRESSURE_SOR ? 8.0 : 1.0);
+        l.cells = cells;
+        l.queued = std::max(mixed ? 3.7 : 3.05, std::max(mixed ? 3.0 + 47.0e-6 * cells : 2.9 + 42.0e-6 * cells,
+                                                        3.0 + (mixed ? 1.2 : 0.6) * pcg2d_queue_pieces(h->nx[i], h->ny[i], h->precision)));
+        l.base = cells <= double(kBlk) ? 5.0 : 11.0 + 0.0095 * std::sqrt(cells);  // one block needs no barrier with others
+        l.work = cells * (mixed ? 14.2e-6 : 16.5e-6) * (plain ? 1.0 : 1.75);
     }
-    return best_first;
+    auto estimate = [&](int from, int to) {  // order[from, to) queued
+        std::vector<char> in(h->n, 0);
+        std::vector<double> busy(h->queue.clusters, 0.0);
+        for (int k = from; k < to; ++k) {
+            in[order[k]] = 1;
+            *std::min_element(busy.begin(), busy.end()) += load[order[k]].its * load[order[k]].queued;
+        }
+        double longest = 0.0, work = 0.0, cells = 0.0;
+        for (int i = 0; i < h->n; ++i)
+            if (!in[i]) {
+                longest = std::max(longest, load[i].its * load[i].base);
+                work += load[i].its * load[i].work;
+                cells += load[i].cells;
+            }
+        return *std::max_element(busy.begin(), busy.end()) + longest + work * (cells > (mixed ? 2.1e6 : 1.05e6) ? 1.35 : 1.0);
+    };
+    const int m = (int)order.size();
+    int from = 0, to = m;
+    double best = estimate(0, m);
+    for (int cut = 1; cut <= m; ++cut)
+        for (const bool largest : {false, true}) {
+            const double t = largest ? estimate(0, m - cut) : estimate(cut, m);
+            if (t < best) {
+                best = t;
+                from = largest ? 0 : cut;
+                to = largest ? m - cut : m;
+            }
+        }
+    return std::vector<int>(order.begin() + from, order.begin() + to);
 }
 
 cudaError_t autotune(FlursysBatchHandle *h) {
@@ -531,7 +555,7 @@ cudaError_t autotune(FlursysBatchHandle *h) {
                 cudaError_t m = cudaMemsetAsync(h->h_pin[i].x, 0, sizeof(double) * h->h_ctl[i].cells, h->stream);
                 if (m != cudaSuccess) return m;
             }
-            batch_prepare_pressure<<<1, kBlk, 0, h->stream>>>(h->ctl, h->pin, h->n, blocks);
+            batch_prepare_pressure<<<1, kBlk, 0, h->stream>>>(h->ctl, h->pin, h->n, blocks, h->queued);
             cudaError_t m = cudaGetLastError();
             if (m == cudaSuccess) m = pcg2d_launch(h->pin, h->n, blocks, h->precision, h->stream);
             return m;
@@ -770,10 +794,12 @@ extern "C" int32_t flursys_cuda_batch_create(const FlursysCudaConfig *configs, i
             }
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->h_ctl[a].cells > h->h_ctl[b].cells; });
         plan();
-        if (e == cudaSuccess && !order.empty() && (int)order.size() < count) {
-            const int first = queue_from(h, order);
-            order.erase(order.begin(), order.begin() + first);
-            if (first > 0) plan();
+        if (e == cudaSuccess && !order.empty()) {
+            const std::vector<int> taken = queue_of(h, order);
+            if (taken.size() < order.size()) {
+                order = taken;
+                plan();
+            }
         }
         for (int i : order) h->h_pin[i].resident = 1;
         h->queued = (int)order.size();

@@ -969,6 +969,10 @@ bool pcg2d_queue_fits(int nx, int ny, bool plain, int precision, size_t *smem) {
     return *smem <= kSmemMax;
 }
 
+int pcg2d_queue_pieces(int nx, int ny, int precision) {
+    return pieces_of(precision, 1, (ny + kMaxCluster - 1) / kMaxCluster, nx);
+}
+
 cudaError_t pcg2d_queue_plan(Pcg2dQueuePlan &plan, int precision, size_t smem, int device) {
     plan = Pcg2dQueuePlan{};
     (void)device;

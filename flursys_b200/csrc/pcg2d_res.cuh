@@ -38,6 +38,8 @@ struct Pcg2dQueuePlan {
 };
 // Whether an instance can be solved by the queue's kernel.
 bool pcg2d_queue_fits(int nx, int ny, bool plain, int precision, size_t *smem);
+// Pieces (32 vectors' room of a row) per warp of its blocks.
+int pcg2d_queue_pieces(int nx, int ny, int precision);
 cudaError_t pcg2d_queue_plan(Pcg2dQueuePlan &plan, int precision, size_t smem, int device);
 // `order`: `count` instance indices (device); `next`: a device counter that is
 // 0 at the launch; instances with resident < 0 are skipped.
