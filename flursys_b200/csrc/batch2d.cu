@@ -456,8 +456,8 @@ float time_ms(FlursysBatchHandle *h, int reps, F fn, cudaError_t *e) {
 // are left to the cooperative launch, or none, or all.
 //
 // Queue: a cluster's iterations one after another. Per iteration, MIXED (F64):
-// 64^2 3.7 (3.1), 256^2 6.0 (5.7), 512^2 15.6; rows of a few cells by pieces per
-// warp (4 x 2000 12.8 and 8.2).
+// 64^2 3.5 (3.1), 256^2 5.4 (5.7), 512^2 13.6; rows of a few cells by pieces per
+// warp (4 x 2000 12 and 8.2).
 // Cooperative launch: its longest instance's two barriers per iteration and the
 // work of all, which share the chip. Per iteration in MIXED one 64^2 11.5,
 // sixteen 13, 256 of them 21; one 512^2 19.7; 32 of 256^2 43, and a third more
@@ -479,8 +479,8 @@ std::vector<int> queue_of(const FlursysBatchHandle *h, const std::vector<int> &o
         Load &l = load[i];
         l.its = side * (h->h_pin[i].solver == FLURSYS_PRESSURE_SOR ? 8.0 : 1.0);
         l.cells = cells;
-        l.queued = std::max(mixed ? 3.7 : 3.05, std::max(mixed ? 3.0 + 47.0e-6 * cells : 2.9 + 42.0e-6 * cells,
-                                                        3.0 + (mixed ? 1.2 : 0.6) * pcg2d_queue_pieces(h->nx[i], h->ny[i], h->precision)));
+        l.queued = std::max(mixed ? 3.5 : 3.05, std::max(2.9 + 42.0e-6 * cells,
+                                                        3.0 + (mixed ? 1.1 : 0.6) * pcg2d_queue_pieces(h->nx[i], h->ny[i], h->precision)));
         l.base = cells <= double(kBlk) ? 5.0 : 11.0 + 0.0095 * std::sqrt(cells);  // one block needs no barrier with others
         l.work = cells * (mixed ? 14.2e-6 : 16.5e-6) * (plain ? 1.0 : 1.75);
     }

@@ -23,14 +23,18 @@
 // x itself is projected once at the end: A annihilates constants, so these
 // shifts are rounding-sized and change no iterate.
 //
-// MIXED: r, q and d are FP32; alpha, beta, the means and 1/diagonal are FP64, r
-// and d are updated in FP64 and rounded as they are stored, and so is every
-// product of the inner products formed and summed. x is FP64, and r is replaced
+// MIXED: r, q and d are FP32; every product of the inner products is formed and
+// summed in FP64; alpha, beta, the means and 1/diagonal are FP64, r and d are
+// updated in FP64 and rounded as they are stored. x is FP64, and r is replaced
 // by the FP64 b - A x every replace_every iterations and before convergence is
 // accepted (d then exchanges M r_old for M r_new, and the operator pass is
-// repeated). (With scalars, weights and updates in FP32 an iteration on 509 x
-// 331 took 5.5 us instead of 5.9, and a solve to 1e-12 2761 of them instead of
-// 2563.)
+// repeated). The queue's kernel, whose x takes half of the registers, applies the
+// scalars and weights rounded to FP32, the same alpha to x and r. Against 64
+// bits, as multiples of the streaming kernel's pressure errors: FP32 scalars 1.24
+// +- 0.07 for single cavities at 3e-11, where FP64 ones give 1.05, but 0.6 to 1.1
+// for batches, where FP64 ones give 1.2 (they stop the solves 4% sooner) and took
+// 8 to 15% longer per iteration (a cluster 6%, the grid on 509 x 331 7%, for 7%
+// fewer iterations).
 //
 // What bounds it: latency. On small grids that of the block reduction, the
 // exchange and the scalars' chain; on large ones also the passes', two warps per
@@ -54,6 +58,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "pcg2d_res.cuh"
 
@@ -63,15 +68,18 @@ namespace {
 
 __device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double vfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double vadd(double a, double b) { return __dadd_rn(a, b); }
 // r - alpha q less its mean, and M r + shift + beta d, as they are stored: the
-// owner of a cell and the halo copies of it form the same bits.
-template <typename V>
-__device__ __forceinline__ V next_r(double alpha, V q, V r, double mean) {
-    return V(__dadd_rn(__fma_rn(-alpha, double(q), double(r)), -mean));
+// owner of a cell and the halo copies of it form the same bits. S: the type of the
+// scalars and of the arithmetic.
+template <typename S, typename V>
+__device__ __forceinline__ V next_r(S alpha, V q, V r, S mean) {
+    return V(vadd(vfma(-alpha, S(q), S(r)), -mean));
 }
-template <typename V>
-__device__ __forceinline__ V next_d(double beta, V d, V r, double inv, double shift) {
-    return V(__fma_rn(beta, double(d), __fma_rn(double(r), inv, shift)));
+template <typename S, typename V>
+__device__ __forceinline__ V next_d(S beta, V d, V r, S inv, S shift) {
+    return V(vfma(beta, S(d), vfma(S(r), inv, shift)));
 }
 
 enum : unsigned { kE = 1, kW = 2, kN = 4, kS = 8, kFluid = 16 };
@@ -123,7 +131,13 @@ struct Res2dGroup<T, true> {
 // 1 / diagonal by coupling bits; 0 marks a row that is not fluid.
 struct Res2dTable {
     double inv[32];
+    float inv32[32];  // the same where they are FP32 numbers
 };
+template <typename S>
+__device__ __forceinline__ S weight_of(const Res2dTable &t, unsigned bits) {
+    if constexpr (sizeof(S) == 4) return t.inv32[bits];
+    else return t.inv[bits];
+}
 
 // What warp 0 hands the block after an iteration's reduction.
 enum : int { kStep = 0, kStop = 1, kRefresh = 2, kFail = 3 };
@@ -160,6 +174,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
     constexpr int W = kVec<V>, U = 4 / W;  // cells per vector, vectors per trip
     constexpr int XV = (XN + W - 1) / W;   // vectors of x in registers
     constexpr int NW = T / 32;
+    using S = std::conditional_t<XN == 0, double, V>;  // of the scalars as they are applied
     const int nx = in.nx, ny = in.ny, tid = threadIdx.x, lane = tid & 31;
     const int rows = (ny + grp.nb - 1) / grp.nb;
     const int j0 = min(grp.rank * rows, ny), nr = min(rows, ny - j0);
@@ -189,7 +204,8 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
 
     if (tid < 32) {  // 1 / diagonal by coupling bits; 0 marks a row that is not fluid
         const double dg = double((tid & 1) + ((tid >> 1) & 1)) * in.idx2 + double(((tid >> 2) & 1) + ((tid >> 3) & 1)) * in.idy2;
-        tab.inv[tid] = (tid & kFluid) ? (dg > 0.0 ? 1.0 / dg : 1.0) : 0.0;
+        tab.inv[tid] = (tid & kFluid) ? (dg > 0.0 ? double(S(1.0 / dg)) : 1.0) : 0.0;
+        tab.inv32[tid] = float(tab.inv[tid]);
     }
     for (int k = tid; k < (int)cpad + 2 * P + 2 * W; k += T) ds[k] = V(0);
     for (int k = tid; k < (int)cpad; k += T) rs[k] = qs[k] = V(0);
@@ -579,7 +595,8 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
             continue;
         }
         replaced = false;
-        const double alpha = sc.alpha, mr = sc.mr, beta = sc.beta, shift = sc.shift, md = sc.md;
+        const S alpha = S(sc.alpha), mr = S(sc.mr), beta = S(sc.beta), shift = S(sc.shift);
+        const double ax = double(alpha), md = sc.md;
         if constexpr (XN > 0) {  // a vector of x at a time; values behind a row are never used
             Walk w = first();
             asm volatile("" : "+r"(w.row), "+r"(w.strip));
@@ -590,7 +607,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                     V dc[W];
                     ldv(dc0 + w.row * P + v * W, dc);
 #pragma unroll
-                    for (int k = 0; k < W; ++k) xr[u * W + k] = fma(alpha, double(dc[k]) - md, xr[u * W + k]);
+                    for (int k = 0; k < W; ++k) xr[u * W + k] = fma(ax, double(dc[k]) - md, xr[u * W + k]);
                 }
                 next(w);
             }
@@ -614,21 +631,21 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                 if (v[u] < 0) continue;
                 const int i = v[u] * W, o = row[u] * P + i;
                 V dn[W];
-                double inv[W];
+                S inv[W];
                 unsigned b[W];
                 const unsigned rb = row_bits(row[u]);
-                const double ii = tab.inv[rb | kE | kW];
+                const S ii = weight_of<S>(tab, rb | kE | kW);
 #pragma unroll
                 for (int k = 0; k < W; ++k) {
                     b[k] = PLAIN ? 31u : (unsigned)bs[o + k];
-                    inv[k] = PLAIN ? ii : tab.inv[b[k]];
+                    inv[k] = PLAIN ? ii : weight_of<S>(tab, b[k]);
                 }
                 const bool edge = v[u] == 0 || v[u] == nvec - 1;
                 if (PLAIN && edge) {
 #pragma unroll
                     for (int k = 0; k < W; ++k) {
                         b[k] = i + k < nx ? 31u : 0u;
-                        if (i + k < nx) inv[k] = tab.inv[rb | col_bits(i + k)];
+                        if (i + k < nx) inv[k] = weight_of<S>(tab, rb | col_bits(i + k));
                     }
                 }
                 if (XN == 0) {
@@ -636,8 +653,8 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
                     for (int k = 0; k < W; k += 2) {  // x of two cells per 16-byte access
                         double2 *xp = reinterpret_cast<double2 *>(xs + o + k);
                         double2 xv = *xp;
-                        xv.x = fma(alpha, double(dc[u][k]) - md, xv.x);
-                        xv.y = fma(alpha, double(dc[u][k + 1]) - md, xv.y);
+                        xv.x = fma(ax, double(dc[u][k]) - md, xv.x);
+                        xv.y = fma(ax, double(dc[u][k + 1]) - md, xv.y);
                         *xp = xv;
                     }
                 }
@@ -669,7 +686,7 @@ __device__ __forceinline__ bool res2d_solve(const Pcg2dInstance &in, typename Re
         each_halo([&](int h, V &d, V qv) {
             const V hn = next_r(alpha, qv, hr[h], mr);
             hr[h] = hn;
-            d = next_d(beta, d, hn, tab.inv[hb[h]], shift);
+            d = next_d(beta, d, hn, weight_of<S>(tab, hb[h]), shift);
         });
         ++it;
         ++since;
