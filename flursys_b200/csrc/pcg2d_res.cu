@@ -38,8 +38,8 @@
 //
 // What bounds it: latency. On small grids that of the block reduction, the
 // exchange and the scalars' chain; on large ones also the passes', two warps per
-// scheduler (four in the queue) that keep issue slots 26% (52%) busy and wait on
-// shared memory, conversions and barriers. A lane takes 16 bytes
+// scheduler (four in the queue) that keep issue slots 25% (55%) busy and wait on
+// L2, shared memory and barriers. A lane takes 16 bytes
 // of a row at a time, and without solid or outlet cells the direction's ghost
 // cells hold the wall cell's own value, so that the operator has no boundary
 // case (a pass that derived each cell's position and couplings spent 240

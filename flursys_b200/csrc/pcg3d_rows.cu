@@ -22,8 +22,8 @@
 // What bounds it: latency. On small grids the round (partials and faces through
 // L2 or, in a cluster, through distributed shared memory); on large ones four
 // warps per scheduler that wait on shared memory, L2, their own chains and the
-// block's barriers: at 128^3 in MIXED issue slots are 43% busy, shared memory
-// 35%, the conversions' unit 10%, FP64 6%. DRAM sees the pressure only at the
+// block's barriers: at 128^3 in MIXED issue slots are 42% busy, shared memory
+// 35%, the conversions' unit 11%, FP64 6%. DRAM sees the pressure only at the
 // residual replacements. Per iteration, against the graph-driven form:
 // 75 x 62 x 51 F64 22.5 -> 6.1 us, 64^3 MIXED 20 -> 4.6, 100^3 F64 39 -> 13.6,
 // 128^3 MIXED 30 -> 16.3 (the tile-resident form of pcg3d_res.cu: 20).
