@@ -33,8 +33,8 @@
 // bits, as multiples of the streaming kernel's pressure errors: FP32 scalars 1.24
 // +- 0.07 for single cavities at 3e-11, where FP64 ones give 1.05, but 0.6 to 1.1
 // for batches, where FP64 ones give 1.2 (they stop the solves 4% sooner) and took
-// 8 to 15% longer per iteration (a cluster 6%, the grid on 509 x 331 7%, for 7%
-// fewer iterations).
+// 8 to 15% longer per iteration (a cluster 6%, the grid on 640 x 480 8%, at up to
+// 7% fewer iterations).
 //
 // What bounds it: latency. On small grids that of the block reduction, the
 // exchange and the scalars' chain; on large ones also the passes', two warps per
@@ -824,8 +824,11 @@ const void *res_fn(int precision, int v) {
 }
 int variant_threads(int v) { return v == 0 ? 256 : 512; }
 // Most pieces (32 vectors of a row) per warp with 256 threads: a block
-// reduction of 8 warps is the shorter one, more work per warp the longer.
-constexpr int kSmallPieces = 2;
+// reduction of 8 warps is the shorter one, more work per warp the longer. In
+// MIXED, whose updates convert to FP64 and back, two pieces take longer than
+// twice the warps' reduction (256 and 512 threads, us per iteration: 150 x 120 3.8
+// and 3.5, 400 x 300 5.8 and 4.9, 509 x 331 5.9 and 5.1, 700 x 200 6.4 and 5.5).
+int small_pieces(int precision) { return precision == FLURSYS_PRECISION_MIXED ? 1 : 2; }
 // The queue's kernel keeps x in registers: pieces per warp of 512 threads.
 constexpr int kQueuePieces = 8;
 int pieces_of(int precision, int v, int rows, int nx) {
@@ -890,7 +893,7 @@ cudaError_t pcg2d_res_plan(Pcg2dResPlan &plan, int nx, int ny, bool plain, int p
         plan.smem = cluster ? smem_of<true>(precision, false, rows, nx, plain) : smem_of<false>(precision, false, rows, nx, plain);
         if (plan.smem <= kSmemMax) {
             plan.cluster = cluster;
-            plan.variant = pieces_of(precision, 0, rows, nx) <= kSmallPieces ? 0 : 1;
+            plan.variant = pieces_of(precision, 0, rows, nx) <= small_pieces(precision) ? 0 : 1;
             plan.nblocks = (ny + rows - 1) / rows;
             return true;
         }
