@@ -58,13 +58,15 @@ def test_no_room_for_the_resident_records(oracle, monkeypatch, case):
     torch.cuda.empty_cache()
     room = plain + 10 * MB
     filler = torch.empty(_free() - room, dtype=torch.uint8, device="cuda")
-    assert plain + 4 * MB <= _free() <= resident - 4 * MB
-    h = _Handle(cfg)
-    h.step(1)
-    p = h.download(field)
-    h.close()
-    del filler
-    torch.cuda.empty_cache()
+    try:
+        assert plain + 4 * MB <= _free() <= resident - 4 * MB
+        h = _Handle(cfg)
+        h.step(1)
+        p = h.download(field)
+        h.close()
+    finally:  # the other tests need the memory
+        del filler
+        torch.cuda.empty_cache()
     assert np.array_equal(p, ref)  # the streaming kernel's result
 
 
